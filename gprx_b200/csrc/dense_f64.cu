@@ -59,68 +59,6 @@ GemmParams gemm_params(int M, int N, int K, const double* A, long long lda, cons
 // ---------------------------------------------------------------------------
 // diagonal block: factor and invert in shared memory
 // ---------------------------------------------------------------------------
-constexpr int DIAG_THREADS = 256;
-
-__device__ void blk_load_lower(double* s, int ls, const double* A, long long lda, long long k0, int nb) {
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    int i = e % nb, j = e / nb;
-    s[i + j * ls] = (i >= j) ? A[(k0 + i) + (k0 + j) * lda] : 0.0;
-  }
-  __syncthreads();
-}
-
-// Unblocked right-looking LLT of the nb×nb lower block in shared memory.
-// Returns the first failing column, or -1.
-__device__ int blk_potf2(double* s, int ls, int nb) {
-  __shared__ int fail;
-  if (threadIdx.x == 0) fail = -1;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int j = 0; j < nb; ++j) {
-    if (threadIdx.x == 0) {
-      double dj = s[j + j * ls];
-      if (!(dj > 0.0)) fail = j;
-      else s[j + j * ls] = sqrt(dj);
-    }
-    __syncthreads();
-    if (fail >= 0) return fail;
-    double ljj = s[j + j * ls];
-    for (int i = j + 1 + threadIdx.x; i < nb; i += blockDim.x) s[i + j * ls] = s[i + j * ls] / ljj;
-    __syncthreads();
-    for (int c = j + 1 + warp; c < nb; c += nw) {
-      double lc = s[c + j * ls];
-      for (int i = c + lane; i < nb; i += 32) s[i + c * ls] = fma(-s[i + j * ls], lc, s[i + c * ls]);
-    }
-    __syncthreads();
-  }
-  return -1;
-}
-
-// In-place inverse of the lower nb×nb triangle (LAPACK trti2 order: columns
-// from the right, each a product with the already inverted trailing block).
-__device__ void blk_trti2(double* s, int ls, int nb, bool unit, double* tmp) {
-  for (int j = nb - 1; j >= 0; --j) {
-    double inv = unit ? 1.0 : 1.0 / s[j + j * ls];
-    for (int i = j + 1 + threadIdx.x; i < nb; i += blockDim.x) tmp[i] = s[i + j * ls];
-    __syncthreads();
-    for (int i = j + 1 + threadIdx.x; i < nb; i += blockDim.x) {
-      double v = 0.0;
-      for (int c = j + 1; c <= i; ++c) v = fma(s[i + c * ls], tmp[c], v);
-      s[i + j * ls] = -v * inv;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) s[j + j * ls] = inv;
-    __syncthreads();
-  }
-}
-
-__device__ void blk_store_full(double* dst, int ldd, const double* s, int ls, int nb) {
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    int i = e % nb, j = e / nb;
-    dst[i + j * ldd] = (i >= j) ? s[i + j * ls] : 0.0;
-  }
-}
-
 // Programmatic dependent launch on the factor's chain: a chain kernel first
 // waits for its predecessor in the stream to complete (its writes visible),
 // then lets its own dependent start launching, so the launch of the next
@@ -141,20 +79,44 @@ __global__ void __launch_bounds__(FD_THREADS) potrf_diag_kernel(double* A, long 
   if (f >= 0 && threadIdx.x == 0) dev_fail(st, GPRX_CHOLESKY_FAILED, k0 + f);
 }
 
-__global__ void __launch_bounds__(DIAG_THREADS) tri_inv_blocks_kernel(const double* L, long long ld, int n,
-                                                                       bool unit, double* linv, DevStatus* st) {
-  extern __shared__ double s[];
+// Inverse of one diagonal block per CTA, in the layout and with the tiles of
+// the factor's diagonal step: the 16×16 leaf inverses in parallel, then block
+// row q of X as X_qq (−L_{q,<q} X_{<q,<q}) on DMMA, two barriers a row.
+// Latency-bound (eight rows in sequence, one CTA a block); the column by
+// column form it replaces took 233 µs for the 16 blocks of n = 2000.
+__global__ void __launch_bounds__(FD_THREADS) tri_inv_blocks_kernel(const double* L, long long ld, int n, bool unit,
+                                                                    double* linv, DevStatus* st) {
+  extern __shared__ __align__(16) double smem[];
   if (dev_failed(st)) return;
-  long long k0 = (long long)blockIdx.x * NB;
-  int nb = (int)min((long long)NB, n - k0);
-  const int ls = nb + 1;
-  double* tmp = s + nb * ls;
-  blk_load_lower(s, ls, L, ld, k0, nb);
-  blk_trti2(s, ls, nb, unit, tmp);
-  blk_store_full(linv + (long long)blockIdx.x * NB * NB, NB, s, ls, nb);
+  double* s = smem;
+  double* tmp = s + NB_DIAG * FLS;
+  double* rinv = tmp + TMP_DOUBLES;
+  const int tid = threadIdx.x, warp = tid >> 5, nw = FD_THREADS >> 5;
+  const long long k0 = (long long)blockIdx.x * NB;
+  const int nb = (int)min((long long)NB, n - k0), np = (nb + LF - 1) / LF, npad = np * LF;
+  for (int e = tid; e < npad * npad; e += FD_THREADS) {
+    const int i = e % npad, j = e / npad;
+    if (i < j) continue;
+    const bool in = i < nb;  // j ≤ i
+    cp_async8(s + i + j * FLS, in ? L + (k0 + i) + (k0 + j) * ld : L, in);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int i = tid; i < npad; i += FD_THREADS) rinv[i] = (unit || i >= nb) ? 1.0 : 1.0 / s[i + i * FLS];
+  __syncthreads();
+  for (int q = warp; q < np; q += nw) leaf16_inverse(s, q, rinv);
+  __syncthreads();
+  for (int q = 1; q < np; ++q) {
+    for (int t = warp; t < 2 * q; t += nw) inv_t_tile(s, tmp, q, t);
+    __syncthreads();
+    for (int t = warp; t < 2 * q; t += nw) inv_x_tile(s, tmp, q, t);
+    __syncthreads();
+  }
+  double* out = linv + (long long)blockIdx.x * NB * NB;
+  for (int t = warp; t < (NB_DIAG / LF) * 4; t += nw) store_x_part(s, out, nb, t / 4, t % 4, 4);
 }
 
-static size_t diag_smem(int nb) { return (size_t)(nb * (nb + 1) + nb) * sizeof(double); }
 static size_t fast_diag_smem(int nb) { (void)nb; return diag_block_smem(); }
 
 static cudaError_t diag_attrs() {
@@ -163,7 +125,8 @@ static cudaError_t diag_attrs() {
   cudaError_t e = cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)fast_diag_smem(NB));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(tri_inv_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem(NB));
+  e = cudaFuncSetAttribute(tri_inv_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)fast_diag_smem(NB));
   if (e != cudaSuccess) return e;
   done = true;
   return cudaSuccess;
@@ -464,7 +427,7 @@ cudaError_t tri_inv_blocks(const double* L, long long ld, int n, bool unit, doub
   CK(diag_attrs());
   int nblk = ceil_div(n, NB);
   if (nblk == 0) return cudaSuccess;
-  GPRX_LAUNCH(tri_inv_blocks_kernel, nblk, DIAG_THREADS, diag_smem(min(n, NB)), s, L, ld, n, unit, linv, st);
+  GPRX_LAUNCH(tri_inv_blocks_kernel, nblk, FD_THREADS, fast_diag_smem(NB), s, L, ld, n, unit, linv, st);
   return cudaGetLastError();
 }
 
@@ -664,6 +627,12 @@ cudaError_t lauum_lower(const double* X, long long ldx, int n, double* C, long l
 
 cudaError_t trsm_lower(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
                        DevStatus* st, cudaStream_t s) {
+  if (tri_solve_few(n, q)) return tri_solve(L, ld, n, linv, B, ldb, q, false, st, s);
+  return trsm_lower_wide(L, ld, n, linv, B, ldb, q, st, s);
+}
+
+cudaError_t trsm_lower_wide(const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+                            int q, DevStatus* st, cudaStream_t s) {
   for (int k0 = 0; k0 < n; k0 += NB) {
     int nbk = min(NB, n - k0);
     const double* lk = linv + (long long)(k0 / NB) * NB * NB;
@@ -681,6 +650,7 @@ cudaError_t trsm_lower(const double* L, long long ld, int n, const double* linv,
 
 cudaError_t trsm_lower_t(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
                          DevStatus* st, cudaStream_t s) {
+  if (tri_solve_few(n, q)) return tri_solve(L, ld, n, linv, B, ldb, q, true, st, s);
   int nblk = ceil_div(n, NB);
   for (int kb = nblk - 1; kb >= 0; --kb) {
     int k0 = kb * NB;

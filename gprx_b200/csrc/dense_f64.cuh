@@ -60,11 +60,24 @@ cudaError_t lauum_lower(const double* X, long long ldx, int n, double* C, long l
 
 struct EmuWork;
 
-// B (n×q, ldb) := L⁻¹ B   /   := L⁻ᵀ B, with L's diagonal block inverses.
+// B (n×q, ldb) := L⁻¹ B   /   := L⁻ᵀ B, with L's diagonal block inverses:
+// tri_solve where tri_solve_few says so, else (trsm_lower_wide) two GEMMs per
+// 128 rows.
 cudaError_t trsm_lower(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
                        DevStatus* st, cudaStream_t s);
 cudaError_t trsm_lower_t(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
                          DevStatus* st, cudaStream_t s);
+
+cudaError_t trsm_lower_wide(const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+                            int q, DevStatus* st, cudaStream_t s);
+
+// The same two solves (trans: L⁻ᵀ) with few right-hand sides in one launch of
+// thread-block clusters (tri_solve.cu); a column's bits do not depend on q.
+// prefix (one right-hand side): prefix[i + s·ldp] receives the sum of L(i, :)
+// x over the columns of the first s + 1 blocks, for the rows below block s.
+bool tri_solve_few(long long n, long long q);
+cudaError_t tri_solve(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
+                      bool trans, const DevStatus* st, cudaStream_t s, double* prefix = nullptr, long long ldp = 0);
 
 // The same two solves for wide B (q ≫ n) by recursive halving: X1 from the
 // top half, one rank-n1 update B2 −= L21 X1 (L21ᵀ X2 for the transpose), then

@@ -829,8 +829,10 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
   const int qc_max = (int)std::max<long long>(1, std::min<long long>((long long)q, (1LL << 27) / std::max(n, 1)));
   if (qbuf.ensure((size_t)ld * qc_max) != cudaSuccess || qx.ensure((size_t)qc_max * (d + 3)) != cudaSuccess)
     return set_error(GPRX_OUT_OF_MEMORY, "predict scratch");
-  HostPinned<double> hm;
-  GPRX_CUDA_TRY(hm.ensure(2 * (size_t)qc_max));
+  GPRX_CUDA_TRY(pred_h.ensure(2 * (size_t)qc_max));
+  double* const hm = pred_h.p;
+  // one route for the whole call: a query's bits do not depend on its chunk
+  const bool few = tri_solve_few(n, (long long)q);
   const double kss = kern.diag_value();
   for (uint64_t c0 = 0; c0 < q; c0 += qc_max) {
     int qc = (int)std::min<uint64_t>(qc_max, q - c0);
@@ -842,17 +844,18 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
                                     cudaMemcpyHostToDevice, stream));
     GPRX_CUDA_TRY(fill_cross(kern, x.p, cap, n, xq, qc, qc, qbuf.p, ld, status.p, stream));
     GPRX_CUDA_TRY(gemv_t(qbuf.p, ld, n, qc, false, alpha.p, mdev, status.p, stream));
-    GPRX_CUDA_TRY(trsm_lower(A.p, ld, n, linv.p, qbuf.p, ld, qc, status.p, stream));
+    if (few) GPRX_CUDA_TRY(tri_solve(A.p, ld, n, linv.p, qbuf.p, ld, qc, false, status.p, stream));
+    else GPRX_CUDA_TRY(trsm_lower_wide(A.p, ld, n, linv.p, qbuf.p, ld, qc, status.p, stream));
     GPRX_CUDA_TRY(col_sumsq(qbuf.p, ld, n, qc, online ? tmpv.p : nullptr, quad, status.p, stream));
     finish_var_kernel<<<ceil_div(qc, 256), 256, 0, stream>>>(quad, qc, kss, noise(), kind, vdev, status.p);
     count_launch();
-    GPRX_CUDA_TRY(cudaMemcpyAsync(hm.p, mdev, sizeof(double) * qc, cudaMemcpyDeviceToHost, stream));
-    GPRX_CUDA_TRY(cudaMemcpyAsync(hm.p + qc_max, vdev, sizeof(double) * qc, cudaMemcpyDeviceToHost, stream));
+    GPRX_CUDA_TRY(cudaMemcpyAsync(hm, mdev, sizeof(double) * qc, cudaMemcpyDeviceToHost, stream));
+    GPRX_CUDA_TRY(cudaMemcpyAsync(hm + qc_max, vdev, sizeof(double) * qc, cudaMemcpyDeviceToHost, stream));
     DevStatus ds;
     if ((st = read_status(&ds)) != GPRX_OK) return st;
     if (ds.code != GPRX_OK) return status_to_error(ds, jitter, n, GPRX_STAGE_PREDICT);
-    std::copy(hm.p, hm.p + qc, mean + c0);
-    std::copy(hm.p + qc_max, hm.p + qc_max + qc, var + c0);
+    std::copy(hm, hm + qc, mean + c0);
+    std::copy(hm + qc_max, hm + qc_max + qc, var + c0);
   }
   return GPRX_OK;
 }

@@ -57,6 +57,7 @@ struct ExactState {
   HostPinned<double> res_h;
   HostPinned<DevStatus> status_h;
   DevBuf<double> qbuf, qx;  // predict scratch
+  HostPinned<double> pred_h;
   DevBuf<unsigned char> group_dev;       // grouped-predict staging (this handle leads the group)
   HostPinned<unsigned char> group_host;
   // mixed precision: the inverse's products emulated on the int8 tensor cores
@@ -132,6 +133,8 @@ struct ExactState {
   // op leaves the LDLT, α and the jitter as they were
   // (with_llt_view, src/gpr/online.rs:1151-1185).
   DevBuf<double> ldlt_keep, alpha_keep;
+  DevBuf<double> spare_A, spare_x, spare_y;  // a delete writes here, then swaps
+  DevBuf<double> r1;                         // its vectors: p, β, new D, per-block sums
   gprx_status with_llt_view(const std::function<gprx_status()>& op);
   gprx_status online_insert(const double* xnew, double ynew, uint64_t* id);
   gprx_status online_delete(uint64_t id);

@@ -10,10 +10,9 @@
 // (src/linalg/ldlt.rs:146-204) and IdRegistry (src/points.rs:76-190).
 //
 // The row/column delete is restated as the rank-1 LDLT update of the
-// trailing block by D_k l_k l_kᵀ (Gill, Golub, Murray & Saunders 1974, C1),
-// blocked 32 columns at a time: one warp runs the 32-step scalar recurrence
-// on the block's own rows, then every thread applies the 32 column updates to
-// its rows below.
+// trailing block by D_k l_k l_kᵀ (Gill, Golub, Murray & Saunders 1974, C1):
+// p = L⁻¹ w, the scalars in closed form from one running sum, then every entry
+// from the sum of its own row up to its column block.
 
 #include <algorithm>
 #include <cmath>
@@ -52,86 +51,82 @@ __global__ void ldlt_border_kernel(double* A, long long ld, int n, const double*
   }
 }
 
-// Rank-1 update L D Lᵀ + a·w wᵀ of the trailing block starting at row/col r0
-// (size m), with w = L[r0.., idx] and a = D_idx.  Single CTA, 1024 threads.
-constexpr int R1_THREADS = 256;
-__global__ void __launch_bounds__(R1_THREADS) ldlt_rank1_kernel(double* A, long long ld, int r0, int m, int idx,
-                                                                 DevStatus* st) {
-  __shared__ double P[32], Bt[32];
-  __shared__ double a_sh;
+// Rank-1 update L D Lᵀ + a·w wᵀ of the trailing block (rows r0 .. n−1, w =
+// L[r0.., idx], a = D_idx) with p = L⁻¹ w: the recurrence
+//   D'_j = D_j + a_j p_j²,  β_j = a_j p_j / D'_j,  a_{j+1} = a_j D_j / D'_j
+// has 1/a_{j+1} = 1/a_j + p_j²/D_j, so every a_j comes from one running sum of
+// non-negative terms.  Rows count from row0 (a multiple of the block width;
+// p is zero before r0).  One CTA: a thread sums a run of rows, the runs are
+// scanned in shared memory.
+constexpr int R1_THREADS = 1024;
+__global__ void __launch_bounds__(R1_THREADS) ldlt_rank1_scan_kernel(const double* A, long long ld, int row0, int r0,
+                                                                     int n, int idx, const double* p, double* beta,
+                                                                     double* dnew, const DevStatus* st) {
+  __shared__ double run[R1_THREADS];
   if (dev_failed(st)) return;
-  // w lives in column idx of A (rows r0..r0+m−1); it is updated in place
-  // there (that column is dropped afterwards).
-  double* w = A + (long long)idx * ld;
-  if (threadIdx.x == 0) a_sh = A[idx + (long long)idx * ld];
+  const int tid = threadIdx.x, per = (n - r0 + R1_THREADS - 1) / R1_THREADS;
+  const int lo = min(n, r0 + tid * per), hi = min(n, lo + per);
+  double acc = 0.0;
+  for (int i = lo; i < hi; ++i) acc += p[i - row0] * p[i - row0] / A[i + (long long)i * ld];
+  run[tid] = acc;
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int jb = 0; jb < m; jb += 32) {
-    int nbk = min(32, m - jb);
-    if (warp == 0) {
-      // lane owns row r = r0 + jb + lane of the block
-      int r = r0 + jb + lane;
-      bool live = lane < nbk;
-      double wr = live ? w[r] : 0.0;
-      double Lr[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) Lr[c] = (live && c < lane) ? A[r + (long long)(r0 + jb + c) * ld] : 0.0;
-      double a = a_sh;
-      // D of the block's rows, read before any of them is rewritten
-      double dmine = live ? A[r + (long long)r * ld] : 1.0;
-      double dnew_mine = dmine;
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        if (c >= nbk) break;
-        double p = __shfl_sync(0xffffffffu, wr, c);
-        double dj = __shfl_sync(0xffffffffu, dmine, c);
-        double dnew = fma(a * p, p, dj);
-        double beta = p * a / dnew;
-        a = dj * a / dnew;
-        if (lane == c) {
-          P[c] = p;
-          Bt[c] = beta;
-          dnew_mine = dnew;
-        }
-        if (live && lane > c) {
-          wr = fma(-p, Lr[c], wr);
-          Lr[c] = fma(beta, wr, Lr[c]);
-        }
-      }
-      if (live) {
-        w[r] = wr;
-        A[r + (long long)r * ld] = dnew_mine;
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (c < lane) A[r + (long long)(r0 + jb + c) * ld] = Lr[c];
-      }
-      if (lane == 0) a_sh = a;
-    }
+  for (int o = 1; o < R1_THREADS; o *= 2) {
+    const double v = tid >= o ? run[tid - o] : 0.0;
     __syncthreads();
-    for (int rr = jb + nbk + threadIdx.x; rr < m; rr += blockDim.x) {
-      int r = r0 + rr;
-      double wr = w[r];
-      for (int c = 0; c < nbk; ++c) {
-        double* l = A + r + (long long)(r0 + jb + c) * ld;
-        wr = fma(-P[c], *l, wr);
-        *l = fma(Bt[c], wr, *l);
-      }
-      w[r] = wr;
-    }
+    run[tid] += v;
     __syncthreads();
+  }
+  double t = 1.0 / A[idx + (long long)idx * ld] + (tid > 0 ? run[tid - 1] : 0.0);
+  for (int i = lo; i < hi; ++i) {
+    const double pi = p[i - row0], di = A[i + (long long)i * ld], a = 1.0 / t;
+    const double dn = fma(a * pi, pi, di);
+    beta[i - row0] = a * pi / dn;
+    dnew[i - row0] = dn;
+    t += pi * pi / di;
   }
 }
 
-// Out-of-place compaction of the lower triangle without row/column idx.
-__global__ void drop_rowcol_kernel(const double* A, long long lda, int n, int idx, double* B, long long ldb) {
-  long long total = (long long)(n - 1) * (n - 1);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(e % (n - 1)), j = (int)(e / (n - 1));
-    if (i < j) continue;
-    int si = i >= idx ? i + 1 : i, sj = j >= idx ? j + 1 : j;
-    B[i + (long long)j * ldb] = A[si + (long long)sj * lda];
+// B = A without row and column idx, the trailing block updated on the way:
+// thread = row, a CTA walks one 128-column block.  Row r enters the block
+// with w_r less the sum over the blocks before it (prefix) and leaves behind
+// L'_rc = L_rc + β_c w_r column by column.  HBM/L2-bound: the lower triangle
+// is read once and written once (6 µs of 32 MB at n = 2000 out of L2); the
+// single-CTA form took 4.5 ms there, every column through one SM.
+constexpr int DEL_ROWS = 128;
+__global__ void __launch_bounds__(DEL_ROWS) ldlt_delete_kernel(const double* A, long long ld, int n, int idx, int row0,
+                                                               const double* p, const double* beta,
+                                                               const double* dnew, const double* prefix,
+                                                               long long ldp, double* B, long long ldb,
+                                                               const DevStatus* st) {
+  if (dev_failed(st)) return;
+  const int r = blockIdx.x * DEL_ROWS + threadIdx.x, c0 = blockIdx.y * NB;
+  if (r >= n || r == idx || r < c0) return;
+  const int c1 = min(min(n, c0 + NB), r + 1);  // columns [c0, c1) of this row
+  const double* a = A + r;
+  const int rb = r > idx ? r - 1 : r;
+  for (int c = c0; c < min(c1, idx); ++c) B[rb + (long long)c * ldb] = a[(long long)c * ld];
+  if (r < idx) return;
+  int c = max(c0, idx + 1);
+  if (c >= c1) return;
+  double w = a[(long long)idx * ld];
+  if (c0 > row0) w -= prefix[(r - row0) + (long long)((c0 - row0) / NB - 1) * ldp];
+  const int last = min(c1, r);  // strictly below the diagonal
+  for (; c + 8 <= last; c += 8) {
+    double l[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) l[u] = a[(long long)(c + u) * ld];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      w = fma(-p[c + u - row0], l[u], w);
+      B[rb + (long long)(c + u - 1) * ldb] = fma(beta[c + u - row0], w, l[u]);
+    }
   }
+  for (; c < last; ++c) {
+    const double l = a[(long long)c * ld];
+    w = fma(-p[c - row0], l, w);
+    B[rb + (long long)(c - 1) * ldb] = fma(beta[c - row0], w, l);
+  }
+  if (c1 == r + 1) B[rb + (long long)(r - 1) * ldb] = dnew[r - row0];
 }
 
 __global__ void drop_row_kernel(const double* x, long long ldx, int n, int d, int idx, double* out, long long ldo) {
@@ -281,30 +276,44 @@ gprx_status ExactState::online_delete(uint64_t id) {
   int idx = (int)(it - ids.begin());
   gprx_status st;
   if ((st = reset_status()) != GPRX_OK) return st;
-  int m = n - idx - 1;
-  if (m > 0) {
-    ldlt_rank1_kernel<<<1, R1_THREADS, 0, stream>>>(A.p, ld, idx + 1, m, idx, status.p);
-    count_launch();
-  }
-  DevBuf<double> nA, nx, ny;
-  if (nA.alloc((size_t)ld * cap) != cudaSuccess || nx.alloc((size_t)cap * d) != cudaSuccess ||
-      ny.alloc(cap) != cudaSuccess)
+  const int row0 = (idx + 1) / NB * NB, len = n - row0;  // whole blocks from the first trailing row
+  if (spare_A.ensure((size_t)ld * cap) != cudaSuccess || spare_x.ensure((size_t)cap * d) != cudaSuccess ||
+      spare_y.ensure(cap) != cudaSuccess ||
+      r1.ensure((size_t)std::max(len, 1) * (3 + ceil_div(std::max(len, 1), NB))) != cudaSuccess)
     return set_error(GPRX_OUT_OF_MEMORY, "online delete scratch");
-  long long tot = (long long)(n - 1) * (n - 1);
-  int blocks = (int)std::max<long long>(1, std::min<long long>((tot + 255) / 256, 148LL * 16));
-  drop_rowcol_kernel<<<blocks, 256, 0, stream>>>(A.p, ld, n, idx, nA.p, ld);
-  drop_row_kernel<<<ceil_div((long long)(n - 1) * d, 256) + 1, 256, 0, stream>>>(x.p, cap, n, d, idx, nx.p, cap);
-  drop_row_kernel<<<ceil_div(n, 256) + 1, 256, 0, stream>>>(y.p, cap, n, 1, idx, ny.p, cap);
-  count_launch(3);
+  double* p = r1.p;
+  double* beta = p + std::max(len, 0);
+  double* dnew = beta + std::max(len, 0);
+  double* prefix = dnew + std::max(len, 0);
+  if (idx + 1 < n) {
+    if (!linv_ok) {
+      GPRX_CUDA_TRY(tri_inv_blocks(A.p, ld, n, true, linv.p, status.p, stream));
+      linv_ok = true;
+    }
+    // p = L⁻¹ w over the blocks that hold trailing rows, zero before them
+    const int lead = idx + 1 - row0;
+    if (lead > 0) GPRX_CUDA_TRY(cudaMemsetAsync(p, 0, sizeof(double) * lead, stream));
+    GPRX_CUDA_TRY(cudaMemcpyAsync(p + lead, A.p + (idx + 1) + (long long)idx * ld, sizeof(double) * (n - idx - 1),
+                                  cudaMemcpyDeviceToDevice, stream));
+    GPRX_CUDA_TRY(tri_solve(A.p + row0 + (long long)row0 * ld, ld, len, linv.p + (long long)(row0 / NB) * NB * NB, p,
+                            len, 1, false, status.p, stream, prefix, len));
+    GPRX_LAUNCH(ldlt_rank1_scan_kernel, 1, R1_THREADS, 0, stream, A.p, ld, row0, idx + 1, n, idx, p, beta, dnew,
+                status.p);
+  }
+  GPRX_LAUNCH(ldlt_delete_kernel, dim3(ceil_div(n, DEL_ROWS), ceil_div(n, NB)), DEL_ROWS, 0, stream, A.p, ld, n, idx,
+              row0, p, beta, dnew, prefix, (long long)len, spare_A.p, ld, status.p);
+  GPRX_LAUNCH(drop_row_kernel, ceil_div((long long)(n - 1) * d, 256) + 1, 256, 0, stream, x.p, cap, n, d, idx,
+              spare_x.p, cap);
+  GPRX_LAUNCH(drop_row_kernel, ceil_div(n, 256) + 1, 256, 0, stream, y.p, cap, n, 1, idx, spare_y.p, cap);
   DevStatus ds;
   if ((st = read_status(&ds)) != GPRX_OK) return st;
   if (ds.code != GPRX_OK) return status_to_error(ds, 0.0, n, GPRX_STAGE_ONLINE_DELETE);
-  std::swap(A.p, nA.p);
-  std::swap(A.n, nA.n);
-  std::swap(x.p, nx.p);
-  std::swap(x.n, nx.n);
-  std::swap(y.p, ny.p);
-  std::swap(y.n, ny.n);
+  std::swap(A.p, spare_A.p);
+  std::swap(A.n, spare_A.n);
+  std::swap(x.p, spare_x.p);
+  std::swap(x.n, spare_x.n);
+  std::swap(y.p, spare_y.p);
+  std::swap(y.n, spare_y.n);
   y_host.erase(y_host.begin() + idx);
   ids.erase(it);
   n -= 1;
