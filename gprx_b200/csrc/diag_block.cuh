@@ -11,18 +11,19 @@ constexpr int NB_DIAG = 128;
 
 // ---------------------------------------------------------------------------
 // Diagonal block (nb ≤ 128): LLT and the block's inverse X = L⁻¹ in shared
-// memory, one CTA of FD_THREADS threads (warp 0 and seven helper warps).  The
-// block is padded to a multiple of 16 with an identity tail.
+// memory, one CTA of a multiple of 128 and at least 256 threads (FD_THREADS:
+// warp 0 and fifteen helper warps).  The block is padded to a multiple of 16
+// with an identity tail.
 //
 // Left-looking by 16-column blocks p, two barriers per step:
 //   warp 0   : the leaf (p, p) takes panel p−1 (its earlier panels are in),
-//              then its 16×16 LLT in registers (lane = row, pivots by shuffles);
+//              then its 16×16 LLT and inverse in registers (lane = row);
 //   helpers  : column block p below the leaf takes panel p−1; column block
 //              p+1 takes panels 0..p−1 in one product; block row p−1 of X:
-//              X_{p−1,p−1} = L_{p−1,p−1}⁻¹ (one warp), T = L_{p−1,<p−1} X_{<p−1,<p−1},
-//              then X_{p−1,<p−1} = −X_{p−1,p−1} T; and the stores of L column
-//              block p−1 and of X block row p−2 to global memory;
-//   all      : the panel below leaf p by column-oriented substitution.
+//              T = L_{p−1,<p−1} X_{<p−1,<p−1}, then X_{p−1,<p−1} = −X_{p−1,p−1} T;
+//              and the stores of L column block p−1 and of X block row p−2 to
+//              global memory;
+//   all      : the panel below leaf p, A X_ppᵀ.
 // Column block q arrives by its own cp.async group, waited for one step
 // before its first use, so the factor starts while the block still loads.
 //
@@ -30,7 +31,7 @@ constexpr int NB_DIAG = 128;
 // s[j + i·FLS] (the upper triangle), X(i, i) = 1/L_ii on the diagonal once
 // block row i of X is formed (L's diagonal is kept in ldiag for the store).
 // ---------------------------------------------------------------------------
-constexpr int FD_THREADS = 256;
+constexpr int FD_THREADS = 512;
 constexpr int LF = 16;                      // leaf / panel width
 constexpr int FLS = NB_DIAG + 4;            // ld of the block (≡ 4 mod 16: conflict-free fragments)
 constexpr int TLD = 20;                     // ld of T (16 rows; ≡ 4 mod 16)
@@ -57,74 +58,132 @@ __device__ __forceinline__ void mma_tile_smem(double (&c)[4], const double* a, i
   }
 }
 
-// 16×16 leaf LLT, one warp: lanes r and r+16 both hold row r of the block at
-// (off, off) of s in registers; pivots are broadcast by shuffles.  Writes L
-// back to s, 1/L_jj to rinv[off + j] and L_jj to ldiag[off + j].  Returns the
-// failing column or −1 (uniform over the warp).  Out of line: one compact
-// copy for every panel.
+// Reciprocal of a positive normal number: the hardware's 20-bit estimate x0
+// and one cubic step, 1/d = x0 (1 + e + e²) + O(e³) with e = 1 − d·x0 (the
+// geometric series).  e + e² goes to *corr, x0 to *seed: 1/d = seed·(1 + corr).
+__device__ __forceinline__ void rcp_parts(double d, double* seed, double* corr) {
+  double x0;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x0) : "d"(d));
+  const double e = fma(-d, x0, 1.0);
+  *seed = x0;
+  *corr = fma(e, e, e);
+}
+
+// 16×16 leaf LLT and inverse, one warp: lane r < 16 holds row r of the block
+// at (off, off) of s in registers, lane 16 + r row r of the identity, which the
+// same elimination turns into row r of L⁻ᵀ.  Writes L (below the diagonal)
+// back to s, X = L⁻¹ to the transposed slots (X(i, c) to s[c + i·FLS], the
+// diagonal included), 1/L_jj to rinv[off + j] and L_jj to ldiag[off + j].
+// Returns the failing column or −1 (uniform over the warp).
+//
+// Bound by the chain from pivot to pivot on one warp (an FP64 operation is 13
+// cycles there).  The columns stay unscaled (Schur complements a_ij, so
+// A −= a_j a_jᵀ / d_j) until the end: a pivot needs a reciprocal instead of a
+// square root, column j is broadcast before its pivot's reciprocal is known
+// (the entry of the next pivot by a shuffle, the rest through the block itself),
+// and every lane forms the next pivot d' − a²·x0·(1 + corr), so a step is the
+// estimate, four FMAs and one shuffle that overlaps them.  The square
+// roots of all pivots follow in parallel.  2.9 K cycles a leaf alone, 4.3 K
+// beside the helpers' shared-memory loads (5.4 K and 8.6 K with the rsqrt and
+// the scaled column on the chain and no inverse; broadcasts by shuffles only:
+// 3.6 K and 4.9 K; a loop over the pivots instead of straight code: 3.7 K, 5.0 K).
 static __device__ __noinline__ int leaf16_factor(double* s, int off, double* rinv, double* ldiag) {
   const int lane = threadIdx.x & 31, r = lane & 15;
+  const bool low = lane < 16;
+  double* row = s + (off + r) + off * FLS;
   double d[16];
 #pragma unroll
-  for (int c = 0; c < 16; ++c) d[c] = (c <= r) ? s[(off + r) + (off + c) * FLS] : 0.0;
+  for (int c = 0; c < 16; ++c) d[c] = low ? (c <= r ? row[c * FLS] : 0.0) : (c == r ? 1.0 : 0.0);
   int bad = -1;
-  double my_inv = 1.0;
-  // the next pivot is formed first, by its own row from its own entry, so
-  // that the chain from one pivot to the next is a shuffle, the reciprocal
-  // square root, a product and an FMA; the other updates of the step overlap
-  // it (the values are those of the plain order, bit for bit)
-  double piv = __shfl_sync(0xffffffffu, d[0], 0);
+  double mine = 1.0;                     // this row's pivot
+  double dg = low ? row[r * FLS] : 0.0;  // and its diagonal entry, updated by the row itself
+  double piv = __shfl_sync(0xffffffffu, dg, 0);
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    if (!(piv > 0.0) && bad < 0) bad = j;
-    const double rs = rsqrt(fmax(piv, 1e-300));
-    if (r == j) {
-      d[j] = piv * rs;
-      my_inv = rs;
-    } else if (r > j) {
-      d[j] = d[j] * rs;
-    }
-    if (j + 1 < 16) {
-      const double cand = (r == j + 1) ? fma(-d[j], d[j], d[j + 1]) : 0.0;
-      const double nxt = __shfl_sync(0xffffffffu, cand, j + 1);
+    const double v = d[j];
+    const double b1 = __shfl_sync(0xffffffffu, v, j + 1);
+    const double dn = __shfl_sync(0xffffffffu, dg, j + 1);
+    if (low ? r > j : r <= j) row[j * FLS] = v;
+    __syncwarp();
+    double b[16];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        if (c > j) {
-          const double lcj = __shfl_sync(0xffffffffu, d[j], c);
-          if (r >= c) d[c] = fma(-d[j], lcj, d[c]);
-        }
-      }
-      piv = nxt;
+    for (int c = j + 2; c < 16; ++c) b[c] = s[(off + c) + (off + j) * FLS];
+    if (!(piv > 0.0) && bad < 0) bad = j;
+    if (r == j) mine = piv;
+    if (j + 1 < 16) {
+      double x0, corr;
+      rcp_parts(piv, &x0, &corr);
+      const double q = b1 * b1 * x0;
+      piv = fma(-q, corr, dn - q);
+      const double u = v * fma(x0, corr, x0);
+      d[j + 1] = fma(-u, b1, d[j + 1]);
+      dg = fma(-u, v, dg);
+#pragma unroll
+      for (int c = j + 2; c < 16; ++c) d[c] = fma(-u, b[c], d[c]);  // rows above c: never read
     }
   }
   if (bad >= 0) return bad;
-  if (lane < 16) {
-#pragma unroll
-    for (int c = 0; c < 16; ++c)
-      if (c <= r) s[(off + r) + (off + c) * FLS] = d[c];
-    rinv[off + r] = my_inv;
-    ldiag[off + r] = d[r];
+  const double rs = rsqrt(mine);
+  __syncwarp();
+  // column c of both triangles times 1/L_cc
+#pragma unroll 4
+  for (int k = 0; k < 8; ++k) {
+    const int c = 2 * k + (lane >> 4);
+    row[c * FLS] *= __shfl_sync(0xffffffffu, rs, c);
+  }
+  if (low) {
+    rinv[off + r] = rs;
+    ldiag[off + r] = mine * rs;
   }
   __syncwarp();
   return -1;
 }
 
-// One lower 16×8 tile of A[rbeg.., cbeg..] −= Σ_{k<K} L[rbeg+i, k0+k] L[cbeg+j, k0+k]
-// (entries above the diagonal are left alone).
-__device__ __forceinline__ void syrk_tile(double* s, int rbeg, int cbeg, int k0, int K) {
+// The 16 rows from r0 below leaf p (c0 = 16p), one warp: A(rows, c0..) X_ppᵀ.
+__device__ __forceinline__ void panel_rows(double* s, int r0, int c0) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  double c[4] = {0, 0, 0, 0};
-  mma_tile_smem(c, s + rbeg + k0 * FLS, 1, FLS, s + cbeg + k0 * FLS, FLS, 1, K);
-  const int row = rbeg + g, col = cbeg + 2 * t4;
-  if (row >= col) s[row + col * FLS] -= c[0];
-  if (row >= col + 1) s[row + (col + 1) * FLS] -= c[1];
-  if (row + 8 >= col) s[(row + 8) + col * FLS] -= c[2];
-  if (row + 8 >= col + 1) s[(row + 8) + (col + 1) * FLS] -= c[3];
+  double c[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+#pragma unroll
+  for (int kk = 0; kk < LF; kk += 4) {
+    const int k = kk + t4;
+    const double a0 = s[r0 + g + (c0 + k) * FLS], a1 = s[r0 + g + 8 + (c0 + k) * FLS];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // B(k, j) = X(j, k), zero for k > j
+      const int j = 8 * h + g;
+      dmma_16x8x4(c[h], a0, a1, k <= j ? s[c0 + k + (c0 + j) * FLS] : 0.0);
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[r0 + g + ((r & 2) ? 8 : 0) + (c0 + 8 * h + 2 * t4 + (r & 1)) * FLS] = c[h][r];
 }
 
-// 16×8 tiles of a 16-column block from row r0 to npad (tile u: rows
-// r0 + 16·(u/2), columns + 8·(u%2)).
-__device__ __forceinline__ int colblock_tiles(int r0, int npad) { return ((npad - r0) / 16) * 2; }
+// One lower 16×16 tile of A[rbeg.., cbeg..] −= Σ_{k<K} L[rbeg+i, k0+k] L[cbeg+j, k0+k]
+// (entries above the diagonal are left alone; both column halves share the A
+// fragments, so that the loads do not crowd out the leaf's).
+__device__ __forceinline__ void syrk_tile(double* s, int rbeg, int cbeg, int k0, int K) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const double* a = s + rbeg + g + (k0 + t4) * FLS;
+  const double* b = s + cbeg + g + (k0 + t4) * FLS;
+  double c[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+#pragma unroll 4
+  for (int kk = 0; kk < K; kk += 4) {
+    const double a0 = a[kk * FLS], a1 = a[kk * FLS + 8];
+    dmma_16x8x4(c[0], a0, a1, b[kk * FLS]);
+    dmma_16x8x4(c[1], a0, a1, b[kk * FLS + 8]);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int row = rbeg + g + ((r & 2) ? 8 : 0), col = cbeg + 8 * h + 2 * t4 + (r & 1);
+      if (row >= col) s[row + col * FLS] -= c[h][r];
+    }
+}
+
+// 16×16 tiles of a 16-column block from row r0 to npad.
+__device__ __forceinline__ int colblock_tiles(int r0, int npad) { return (npad - r0) / 16; }
 
 // The 16×16 leaf inverse of block q (one warp): lane c computes column c of
 // L_qq⁻¹ by substitution; X(i, c) goes to s[c + i·FLS] (i ≥ c: the diagonal
@@ -225,43 +284,39 @@ __device__ __forceinline__ void cp_async_wait_n(int n) {
   }
 }
 
-// The work of step p that is off warp 0's chain, dealt over nh warps (h =
-// this warp's index among them): inverse block row q = p − 1 (leaf inverse
-// and T, then — after the barrier of the nh warps — X_{q,<q}), the updates
-// of column blocks p (panel p−1, below the leaf) and p+1 (panels 0..p−1),
-// the store of L column block p−1 and of X block row p−2.  With tail, p = np
-// and the whole CTA takes part (barriers are __syncthreads).
+// The work of step p that is off warp 0's chain.  Products (dealt over nh
+// warps, h = this warp's index among them, −1: none): inverse block row
+// q = p − 1 (T, then — after the barrier of the nh warps — X_{q,<q}) and the
+// updates of column blocks p (panel p−1, below the leaf) and p+1 (panels
+// 0..p−1).  Stores (over ns warps, index sh): L column block p−1
+// and X block row p−2.  With tail, p = np and the whole CTA takes part in both
+// (barriers are __syncthreads).
 static __device__ void diag_helpers(double* s, double* tmp, const double* rinv, const double* ldiag, double* A, long long lda,
-                             long long k0, int nb, double* linv, bool vec, int p, int np, int h, int nh, bool tail) {
+                             long long k0, int nb, double* linv, bool vec, int p, int np, int h, int nh, int sh, int ns,
+                             bool tail) {
   const int npad = np * LF, c0 = p * LF, r1 = c0 + LF, q = p - 1;
-  const int n_inv = p >= 1 ? 1 : 0;
+  if (sh >= 0) {
+    const int n_ls = p >= 1 ? 2 : 0, xs_parts = tail ? 4 : 2, n_xs = p >= 2 ? xs_parts : 0;
+    for (int t = sh; t < n_ls + n_xs; t += ns) {
+      if (t < n_ls) store_l_part(s, ldiag, A, lda, k0, nb, vec, q, t);
+      else store_x_part(s, linv, nb, p - 2, t - n_ls, xs_parts);
+    }
+  }
+  if (h < 0) return;
   const int n_t = p >= 2 ? 2 * q : 0;
   const int n_next = (!tail && p >= 1 && p + 1 < np) ? colblock_tiles(r1, npad) : 0;
   const int n_cur = (!tail && p >= 1 && r1 < npad) ? colblock_tiles(r1, npad) : 0;
-  const int n_ls = p >= 1 ? 2 : 0;
-  const int xs_parts = tail ? 4 : 2;
-  const int n_xs = p >= 2 ? xs_parts : 0;
-  const int total = n_inv + n_t + n_next + n_cur + n_ls + n_xs;
+  const int total = n_t + n_next + n_cur;
   for (int t = h; t < total; t += nh) {
     int u = t;
-    if (u < n_inv) { leaf16_inverse(s, q, rinv); continue; }
-    u -= n_inv;
     if (u < n_t) { inv_t_tile(s, tmp, q, u); continue; }
     u -= n_t;
     if (u < n_next) {  // column block p+1, rows from r1, panels 0..p−1
-      const int rbeg = r1 + 16 * (u >> 1), cbeg = r1 + 8 * (u & 1);
-      if (rbeg + 15 >= cbeg) syrk_tile(s, rbeg, cbeg, 0, c0);
+      syrk_tile(s, r1 + 16 * u, r1, 0, c0);
       continue;
     }
-    u -= n_next;
-    if (u < n_cur) {  // column block p below the leaf, panel p−1
-      syrk_tile(s, r1 + 16 * (u >> 1), c0 + 8 * (u & 1), c0 - LF, LF);
-      continue;
-    }
-    u -= n_cur;
-    if (u < n_ls) { store_l_part(s, ldiag, A, lda, k0, nb, vec, q, u); continue; }
-    u -= n_ls;
-    store_x_part(s, linv, nb, p - 2, u, xs_parts);
+    u -= n_next;  // column block p below the leaf, panel p−1
+    syrk_tile(s, r1 + 16 * u, c0, c0 - LF, LF);
   }
   if (p < 2) return;
   if (tail) __syncthreads();
@@ -285,11 +340,10 @@ static __device__ int diag_block_factor_inv(double* A, long long lda, long long 
   const int npad = (nb + LF - 1) / LF * LF, np = npad / LF;
   if (tid == 0) fail = -1;
   // column block q is cp.async group q of every thread (16-byte copies from
-  // the even row at or above the diagonal); blocks 0 and 1 go first alone and
-  // are waited for, the rest then loads during the first steps
+  // the even row at or above the diagonal): blocks 0 and 1 are waited for, the
+  // rest arrives during the first steps
   const bool vec = ((lda & 1) == 0) && ((((unsigned long long)(A + k0 + k0 * lda)) & 15) == 0);
   for (int q = 0; q < np; ++q) {
-    if (q == 2) cp_async_wait<0>();
     for (int j = q * LF + warp; j < q * LF + LF && j < nb; j += nw) {
       if (vec) {
         for (int i = (j & ~1) + 2 * lane; i < nb; i += 64) {
@@ -307,9 +361,10 @@ static __device__ int diag_block_factor_inv(double* A, long long lda, long long 
     cp_async_commit();
   }
   // identity padding (lower part; the copies never reach these entries)
-  for (int j = warp; j < npad; j += nw)
-    for (int i = j + lane; i < npad; i += 32)
-      if (i >= nb || j >= nb) s[i + j * FLS] = (i == j) ? 1.0 : 0.0;
+  if (nb < npad)
+    for (int j = warp; j < npad; j += nw)
+      for (int i = j + lane; i < npad; i += 32)
+        if (i >= nb || j >= nb) s[i + j * FLS] = (i == j) ? 1.0 : 0.0;
   cp_async_wait_n(np - 2);  // column blocks 0 and 1
   __syncthreads();
   for (int p = 0; p < np; ++p) {
@@ -317,35 +372,21 @@ static __device__ int diag_block_factor_inv(double* A, long long lda, long long 
     if (warp == 0) {
       if (p > 0) {  // the leaf's last update: panel p−1
         syrk_tile(s, c0, c0, c0 - LF, LF);
-        syrk_tile(s, c0, c0 + 8, c0 - LF, LF);
         __syncwarp();
       }
       const int f = leaf16_factor(s, c0, rinv, ldiag);
       if (f >= 0 && lane == 0) fail = c0 + f;
     } else {
-      diag_helpers(s, tmp, rinv, ldiag, A, lda, k0, nb, linv, vec, p, np, warp - 1, nw - 1, false);
+      // the warps that share warp 0's scheduler (and its FP64 pipe, which a
+      // DMMA holds for 32 cycles) store; the others multiply
+      const bool store = (warp & 3) == 0;
+      diag_helpers(s, tmp, rinv, ldiag, A, lda, k0, nb, linv, vec, p, np, store ? -1 : warp - 1 - warp / 4,
+                   nw - nw / 4, store ? warp / 4 - 1 : -1, nw / 4 - 1, false);
     }
     __syncthreads();
     if (fail >= 0) break;
-    // panel: rows below the leaf solve X L_ppᵀ = A (32 rows per warp)
-    for (int grp = warp; grp * 32 < npad - r1; grp += nw) {
-      const int row = r1 + grp * 32 + lane;
-      const bool act = row < npad;
-      double a[LF];
-#pragma unroll
-      for (int c = 0; c < LF; ++c) a[c] = act ? s[row + (c0 + c) * FLS] : 0.0;
-#pragma unroll
-      for (int t = 0; t < LF; ++t) {
-        const double x = a[t] * rinv[c0 + t];
-        a[t] = x;
-#pragma unroll
-        for (int j = t + 1; j < LF; ++j) a[j] = fma(-x, s[(c0 + j) + (c0 + t) * FLS], a[j]);
-      }
-      if (act) {
-#pragma unroll
-        for (int c = 0; c < LF; ++c) s[row + (c0 + c) * FLS] = a[c];
-      }
-    }
+    // panel: 16 rows below the leaf per warp
+    for (int r0 = r1 + 16 * warp; r0 < npad; r0 += 16 * nw) panel_rows(s, r0, c0);
     cp_async_wait_n(np - 3 - p);  // column block p+2, used by the next step's helpers
     __syncthreads();
   }
@@ -356,7 +397,7 @@ static __device__ int diag_block_factor_inv(double* A, long long lda, long long 
   }
   // the last block row of X, the last column block of L, the last two block
   // rows of X into linv (all warps)
-  diag_helpers(s, tmp, rinv, ldiag, A, lda, k0, nb, linv, vec, np, np, warp, nw, true);
+  diag_helpers(s, tmp, rinv, ldiag, A, lda, k0, nb, linv, vec, np, np, warp, nw, warp, nw, true);
   __syncthreads();
   // block rows np−1 .. NB_DIAG/16 − 1 (those past the block are zeros)
   for (int t = warp; t < (NB_DIAG / LF - np + 1) * 4; t += nw) store_x_part(s, linv, nb, np - 1 + t / 4, t % 4, 4);
