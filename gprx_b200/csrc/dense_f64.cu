@@ -18,17 +18,57 @@
 
 namespace gprx {
 
-cudaError_t dgemm(bool ta, bool tb, const GemmParams& p, cudaStream_t s, int batch) {
-  if (!ta && !tb) return launch_dgemm<128, 128, 16, 64, 32, 3, false, false>(p, batch, s);
-  if (!ta && tb) return launch_dgemm<128, 128, 16, 64, 32, 3, false, true>(p, batch, s);
-  if (ta && !tb) return launch_dgemm<128, 128, 16, 64, 32, 3, true, false>(p, batch, s);
-  return launch_dgemm<128, 128, 16, 64, 32, 3, true, true>(p, batch, s);
+// 64×64 tiles of four warps (32×32 each, 57 KB, three to four CTAs a SM): one
+// CTA's barriers and epilogue hide behind the others' DMMAs.  Measured against
+// the 128×128 tile of eight warps (one CTA a SM), TF/s: 4096³ 29.7 / 28.0,
+// 512 × 65536 with K = 512 28.8 / 26.2 (A transposed 29.1 / 26.5), A·Aᵀ of
+// 1024 × 65536 split over K 31.1 / 27.7, K = 128 22.3 / 17.3; the sums run over
+// k in the same order for every tile shape.
+template <bool TA, bool TB>
+static cudaError_t dgemm_wide(const GemmParams& p, cudaStream_t s, int batch) {
+  return launch_dgemm<64, 64, 16, 32, 32, 3, TA, TB>(p, batch, s);
 }
 
-cudaError_t dgemm_nn_fill(const GemmParams& p, cudaStream_t s, int batch) {
-  const long long tiles128 = (long long)ceil_div(p.M, 128) * ceil_div(p.N, 128) * batch;
-  if (tiles128 >= 2 * 148) return launch_dgemm<128, 128, 16, 64, 32, 3, false, false>(p, batch, s);
-  return launch_dgemm<64, 64, 16, 32, 16, 3, false, false>(p, batch, s);
+// Output tiles of a product (LOWER_TILES: those not strictly above the diagonal).
+static long long gemm_tiles(const GemmParams& p, int bm, int bn) {
+  const int tm = ceil_div(p.M, bm), tn = ceil_div(p.N, bn);
+  if (!(p.mode & GEMM_LOWER_TILES)) return (long long)tm * tn;
+  long long c = 0;
+  for (int j = 0; j < tn; ++j) {
+    const long long need = p.col0 + (long long)j * bn - p.row0 - (bm - 1);
+    c += std::max(0LL, tm - (need <= 0 ? 0 : (need + bm - 1) / bm));
+  }
+  return c;
+}
+
+// The tile by how many the product has: few tiles leave SMs idle, and the
+// longest k range decides when triangular operands give the tiles different
+// lengths, so below four 64×64 tiles a SM the tile is 32×64 (k chunks of 32 in
+// four stages, eight warps of 16×16: one memory latency a product).  Measured
+// (µs, 128×128 / 64×64 / 32×64): Xᵀ X of n = 512 92 / 37 / 21, n = 1537
+// 264 / 115 / 80, n = 2048 347 / 178 / 153, n = 3000 506 / 377 / 429; a
+// triangular product of n = 256 49 / 21 / 13, n = 1000 176 / 88 / 83, n = 2048
+// 555 / 414 / 443, n = 3000 1390 / 1079 / 1281.
+template <bool TA, bool TB>
+static cudaError_t dgemm_fill(const GemmParams& p, cudaStream_t s, int batch) {
+  const int z = (p.mode & GEMM_SPLIT_K) ? p.splits : batch;
+  if (gemm_tiles(p, 64, 64) * z >= 4 * 148) return dgemm_wide<TA, TB>(p, s, batch);
+  return launch_dgemm<32, 64, 32, 16, 16, 4, TA, TB>(p, batch, s);
+}
+
+cudaError_t dgemm(bool ta, bool tb, const GemmParams& p, cudaStream_t s, int batch) {
+  if (!ta && !tb) return dgemm_fill<false, false>(p, s, batch);
+  if (!ta && tb) return dgemm_fill<false, true>(p, s, batch);
+  if (ta && !tb) return dgemm_fill<true, false>(p, s, batch);
+  return dgemm_fill<true, true>(p, s, batch);
+}
+
+// B := A·B or Aᵀ·B in place (M, K ≤ 128): one tile holds every row of its
+// columns and reads them all before it writes.
+template <bool TA>
+static cudaError_t dgemm_inplace(const GemmParams& p, cudaStream_t s) {
+  if (p.M > 128) return cudaErrorInvalidValue;
+  return launch_dgemm<128, 64, 32, 64, 16, 2, TA, false>(p, 1, s);
 }
 
 GemmParams gemm_params(int M, int N, int K, const double* A, long long lda, const double* B, long long ldb,
@@ -140,6 +180,8 @@ static cudaError_t diag_attrs() {
 
 FactorCtx::~FactorCtx() {
   for (auto e : ev) cudaEventDestroy(e);
+  for (auto e : side)
+    if (e) cudaEventDestroy(e);
   if (aux) cudaStreamDestroy(aux);
   if (aux2) cudaStreamDestroy(aux2);
 }
@@ -155,6 +197,8 @@ cudaError_t FactorCtx::ensure(int nblk) {
     CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     CK(cudaStreamCreateWithPriority(&aux2, cudaStreamNonBlocking, hi));
   }
+  for (auto& e : side)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   while ((int)ev.size() < 3 * nblk + 2) {
     cudaEvent_t e;
     CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -344,14 +388,12 @@ static cudaError_t diag_and_panel(double* A, long long ld, int n, int k0, double
   return cudaGetLastError();
 }
 
-// The bulk trailing update of the look-ahead factor (K = NB) runs on 64×128
-// tiles: half the registers of the 128×128 tile, so two CTAs share an SM and
-// one's copies and epilogue overlap the other's DMMA work, and CTAs short
-// enough that the chain's high-priority kernels get SMs as they retire (no
-// SM is held back).  Measured (FP64 factor probe, n = 4096 / 8192): 2.42 /
-// 10.35 ms, against 2.55 / 11.67 ms with 128×128 tiles capped at 132 CTAs
-// while the trailing block has at most 4096 rows, 3.14 / 11.34 ms with the
-// 64×128 tiles capped at 132 CTAs and 2.53 / 10.40 ms capped at 264.
+// The bulk trailing update of the look-ahead factor (K = NB) runs on 64×64
+// tiles of four warps: CTAs short enough that the chain's high-priority kernels
+// get SMs as they retire (no SM is held back).  Measured (evaluation, n = 1537
+// / 8192): 1.04 / 24.0 ms, against 1.03 / 24.2 ms on 64×128 tiles of eight
+// warps; 128×128 tiles capped at 132 CTAs took 11.67 ms for the n = 8192 factor
+// where the 64×128 tiles took 10.35 ms.
 
 cudaError_t potrf_blocked(double* A, long long ld, int n, double* linv, DevStatus* st, cudaStream_t s,
                           FactorCtx* ctx) {
@@ -414,7 +456,7 @@ cudaError_t potrf_blocked(double* A, long long ld, int n, double* linv, DevStatu
       const double* Pk2 = A + c2 + (long long)k0 * ld;
       GemmParams ps = gemm_params(m, m, NB, Pk2, ld, Pk2, ld, A + c2 + (long long)c2 * ld, ld, -1.0, 1.0, st);
       ps.mode = GEMM_LOWER_TILES;
-      CK((launch_dgemm<64, 128, 16, 32, 32, 3, false, true>(ps, 1, s)));
+      CK((launch_dgemm<64, 64, 16, 32, 32, 3, false, true>(ps, 1, s)));
     }
     CK(cudaEventRecord(Es[k], s));
   }
@@ -456,20 +498,27 @@ cudaError_t set_identity(double* X, long long ld, int n, cudaStream_t s) {
 // blocks gets X21 = −X22 (L21 X11), two batched triangular products with the
 // k-ranges cut to the nonzero triangles.  X's strict upper triangle must be
 // zero on entry (it is never written).  scratch holds ceil(n/2)² doubles.
-__global__ void copy_diag_blocks_kernel(const double* linv, int n, double* X, long long ldx) {
-  long long k0 = (long long)blockIdx.x * NB;
-  int nb = (int)min((long long)NB, n - k0);
-  const double* src = linv + (long long)blockIdx.x * NB * NB;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    int i = e % nb, j = e / nb;
-    X[(k0 + i) + (k0 + j) * ldx] = src[i + j * NB];
-  }
+// One CTA per 16 columns of a block (one CTA per block took 35 µs).
+constexpr int CDB_COLS = 16;
+__global__ void __launch_bounds__(NB) copy_diag_blocks_kernel(const double* linv, int n, double* X, long long ldx) {
+  const long long k0 = (long long)blockIdx.x * NB;
+  const int nb = (int)min((long long)NB, n - k0), i = threadIdx.x, j0 = blockIdx.y * CDB_COLS;
+  if (i >= nb) return;
+  const double* src = linv + (long long)blockIdx.x * NB * NB + i;
+  double* dst = X + (k0 + i) + k0 * ldx;
+#pragma unroll
+  for (int j = j0; j < j0 + CDB_COLS; ++j)
+    if (j < nb) dst[j * ldx] = src[j * NB];
+}
+
+static cudaError_t copy_diag_blocks(const double* linv, int n, double* X, long long ldx, cudaStream_t s) {
+  GPRX_LAUNCH(copy_diag_blocks_kernel, dim3(ceil_div(n, NB), NB / CDB_COLS), NB, 0, s, linv, n, X, ldx);
+  return cudaGetLastError();
 }
 
 cudaError_t trtri_blocked(const double* L, long long ld, int n, const double* linv, double* X, long long ldx,
                           double* scratch, DevStatus* st, cudaStream_t s) {
-  int nblk = ceil_div(n, NB);
-  GPRX_LAUNCH(copy_diag_blocks_kernel, nblk, 256, 0, s, linv, n, X, ldx);
+  CK(copy_diag_blocks(linv, n, X, ldx, s));
   for (long long b = 2LL * NB; b < 2LL * n; b *= 2) {
     long long h = b / 2;
     if (h >= n) break;
@@ -495,7 +544,7 @@ cudaError_t trtri_blocked(const double* L, long long ld, int n, const double* li
       p1.strideA = b + b * ld;
       p1.strideB = b + b * ldx;
       p1.strideC = h2 * h;
-      CK(dgemm_nn_fill(p1, s, (int)cnt));
+      CK(dgemm(false, false, p1, s, (int)cnt));
       // X21 = −X22 · T   (h2 × h, K = h2; X22 lower → k up to the row)
       GemmParams p2 = gemm_params((int)h2, (int)h, (int)h2, X + (s0 + h) + (s0 + h) * ldx, ldx, scratch, h2,
                                   X + (s0 + h) + s0 * ldx, ldx, -1.0, 0.0, st);
@@ -503,7 +552,7 @@ cudaError_t trtri_blocked(const double* L, long long ld, int n, const double* li
       p2.strideA = b + b * ldx;
       p2.strideB = h2 * h;
       p2.strideC = b + b * ldx;
-      CK(dgemm_nn_fill(p2, s, (int)cnt));
+      CK(dgemm(false, false, p2, s, (int)cnt));
     }
   }
   return cudaGetLastError();
@@ -511,8 +560,7 @@ cudaError_t trtri_blocked(const double* L, long long ld, int n, const double* li
 
 cudaError_t trtri_blocked_emu(const double* L, long long ld, int n, const double* linv, double* X, long long ldx,
                               double* scratch, const EmuWork& w, int emu_min, DevStatus* st, cudaStream_t s) {
-  int nblk = ceil_div(n, NB);
-  GPRX_LAUNCH(copy_diag_blocks_kernel, nblk, 256, 0, s, linv, n, X, ldx);
+  CK(copy_diag_blocks(linv, n, X, ldx, s));
   for (long long b = 2LL * NB; b < 2LL * n; b *= 2) {
     long long h = b / 2;
     if (h >= n) break;
@@ -538,14 +586,14 @@ cudaError_t trtri_blocked_emu(const double* L, long long ld, int n, const double
         p1.strideA = b + b * ld;
         p1.strideB = b + b * ldx;
         p1.strideC = h2 * h;
-        CK(dgemm_nn_fill(p1, s, (int)cnt));
+        CK(dgemm(false, false, p1, s, (int)cnt));
         GemmParams p2 = gemm_params((int)h2, (int)h, (int)h2, X + (s0 + h) + (s0 + h) * ldx, ldx, scratch, h2,
                                     X + (s0 + h) + s0 * ldx, ldx, -1.0, 0.0, st);
         p2.mode = GEMM_K_TO_ROW;
         p2.strideA = b + b * ldx;
         p2.strideB = h2 * h;
         p2.strideC = b + b * ldx;
-        CK(dgemm_nn_fill(p2, s, (int)cnt));
+        CK(dgemm(false, false, p2, s, (int)cnt));
         continue;
       }
       for (long long c = 0; c < cnt; ++c) {
@@ -622,7 +670,7 @@ cudaError_t lauum_lower(const double* X, long long ldx, int n, double* C, long l
                         cudaStream_t s) {
   GemmParams p = gemm_params(n, n, n, X, ldx, X, ldx, C, ldc, 1.0, 0.0, st);
   p.mode = GEMM_LOWER_TILES | GEMM_K_FROM_ROW;
-  return dgemm(true, false, p, s);
+  return dgemm_fill<true, false>(p, s, 1);
 }
 
 cudaError_t trsm_lower(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
@@ -638,7 +686,7 @@ cudaError_t trsm_lower_wide(const double* L, long long ld, int n, const double* 
     const double* lk = linv + (long long)(k0 / NB) * NB * NB;
     double* Bk = B + k0;
     GemmParams p1 = gemm_params(nbk, q, nbk, lk, NB, Bk, ldb, Bk, ldb, 1.0, 0.0, st);
-    CK(dgemm(false, false, p1, s));
+    CK(dgemm_inplace<false>(p1, s));
     int rest = n - k0 - nbk;
     if (rest <= 0) break;
     GemmParams p2 = gemm_params(rest, q, nbk, L + (k0 + nbk) + (long long)k0 * ld, ld, Bk, ldb, B + k0 + nbk, ldb,
@@ -659,7 +707,7 @@ cudaError_t trsm_lower_t(const double* L, long long ld, int n, const double* lin
     double* Bk = B + k0;
     // B_k := L_kk⁻ᵀ B_k
     GemmParams p1 = gemm_params(nbk, q, nbk, lk, NB, Bk, ldb, Bk, ldb, 1.0, 0.0, st);
-    CK(dgemm(true, false, p1, s));
+    CK(dgemm_inplace<true>(p1, s));
     if (k0 == 0) break;
     // B_{<k} −= L_{k,<k}ᵀ B_k
     GemmParams p2 = gemm_params(k0, q, nbk, L + k0, ld, Bk, ldb, B, ldb, -1.0, 1.0, st);

@@ -12,11 +12,9 @@ namespace gprx {
 // steps need it ≤ the 128-wide GEMM tile.
 constexpr int NB = 128;
 
-// C = alpha·opA·opB + beta·C with the 128×128 DMMA tile (see gemm_f64.cuh).
+// C = alpha·opA·opB + beta·C on DMMA tiles chosen by their number (see
+// gemm_f64.cuh); C must not alias A or B.
 cudaError_t dgemm(bool ta, bool tb, const GemmParams& p, cudaStream_t s, int batch = 1);
-// A·B (NN) with 64×64 tiles when 128×128 tiles would leave most SMs idle
-// (fewer than two waves); C must not alias A or B.
-cudaError_t dgemm_nn_fill(const GemmParams& p, cudaStream_t s, int batch);
 
 // Small helper building GemmParams.
 GemmParams gemm_params(int M, int N, int K, const double* A, long long lda, const double* B, long long ldb,
@@ -24,12 +22,14 @@ GemmParams gemm_params(int M, int N, int K, const double* A, long long lda, cons
 
 // Side streams and events of the look-ahead factorization (one per handle):
 // aux carries the chain, aux2 the column update's rows below the diagonal
-// block (concurrent with the diagonal block).
+// block (concurrent with the diagonal block).  After the factor, aux is free
+// for work beside the inverse's products (side: events for that).
 struct FactorCtx {
   int device = -1;
   cudaStream_t aux = nullptr;
   cudaStream_t aux2 = nullptr;
   std::vector<cudaEvent_t> ev;
+  cudaEvent_t side[4] = {nullptr, nullptr, nullptr, nullptr};
   ~FactorCtx();
   cudaError_t ensure(int nblk);
 };

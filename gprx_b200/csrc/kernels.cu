@@ -840,14 +840,19 @@ cudaError_t cross_contract(const HostKernel& k, const double* z, long long ldz, 
 }
 
 // grad[p] = scale · Σ_slots(p); grad[n_kernel] = noise_coef · Σ (last slot).
+// A warp per slot, lanes over the blocks (one thread per slot: 51 µs at
+// n = 1537, every partial a memory latency).
+constexpr int FINALIZE_THREADS = 1024;
 __global__ void grad_finalize_kernel(const double* partials, int blocks, int ns, const int* slot_param, int n_kernel,
                                      double scale, double noise_coef, double* grad, const DevStatus* st) {
   __shared__ double tot[64];
   if (dev_failed(st)) return;
-  for (int s = threadIdx.x; s < ns; s += blockDim.x) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int s = threadIdx.x >> 5; s < ns; s += nw) {
     double v = 0.0;
-    for (int b = 0; b < blocks; ++b) v += partials[(long long)b * ns + s];
-    tot[s] = v;
+    for (int b = lane; b < blocks; b += 32) v += partials[(long long)b * ns + s];
+    v = warp_sum(v);
+    if (lane == 0) tot[s] = v;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -864,7 +869,7 @@ __global__ void grad_finalize_kernel(const double* partials, int blocks, int ns,
 cudaError_t grad_finalize(const HostKernel& k, const double* partials, int blocks, const int* slot_param_dev,
                           double scale, double noise_coef, double* grad, DevStatus* st, cudaStream_t s) {
   int ns = grad_slots(k.ard_d);
-  GPRX_LAUNCH(grad_finalize_kernel, 1, 64, 0, s, partials, blocks, ns, slot_param_dev, k.n_params, scale,
+  GPRX_LAUNCH(grad_finalize_kernel, 1, FINALIZE_THREADS, 0, s, partials, blocks, ns, slot_param_dev, k.n_params, scale,
               noise_coef, grad, st);
   return cudaGetLastError();
 }
