@@ -623,7 +623,7 @@ struct BatchState {
   ~BatchState() {
     if (stream) cudaStreamSynchronize(stream);
     if (graph) cudaGraphExecDestroy(graph);
-    if (stream) cudaStreamDestroy(stream);
+    stream_release(stream, false, device);
   }
 
   gprx_status create(const double* xh, const double* yh, const uint64_t* ns, uint64_t np, uint64_t dd,
@@ -688,7 +688,7 @@ gprx_status BatchState::create(const double* xh, const double* yh, const uint64_
   p = n_theta;
   device = opt.device;
   GPRX_CUDA_TRY(cudaSetDevice(device));
-  GPRX_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  GPRX_CUDA_TRY(stream_acquire(&stream, false));
   int sms = 0;
   GPRX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   smem = batch_smem();
@@ -910,6 +910,10 @@ gprx_status BatchState::fit(const double* theta0, const gprx_lbfgs_options* o, d
       this->theta_out.ensure((size_t)nprob * p))
     return set_error(GPRX_OUT_OF_MEMORY, "fit buffers");
   GPRX_CUDA_TRY(cudaMemcpyAsync(zstart.p, zs.data(), sizeof(double) * zs.size(), cudaMemcpyHostToDevice, stream));
+  // the states start at zero, whoever had the memory before: with the history
+  // full, the pair ring reads a slot it has not written (its zero curvature
+  // makes that step restart from steepest descent)
+  GPRX_CUDA_TRY(cudaMemsetAsync(fits.p, 0, sizeof(ProblemFit) * nprob, stream));
   FitArgs fa{};
   fa.fits = fits.p;
   fa.nprob = nprob;

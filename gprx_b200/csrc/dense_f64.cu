@@ -15,6 +15,7 @@
 #include "dense_f64.cuh"
 #include "emu_gemm.cuh"
 #include "diag_block.cuh"
+#include "pool.h"
 
 namespace gprx {
 
@@ -182,21 +183,14 @@ FactorCtx::~FactorCtx() {
   for (auto e : ev) cudaEventDestroy(e);
   for (auto e : side)
     if (e) cudaEventDestroy(e);
-  if (aux) cudaStreamDestroy(aux);
-  if (aux2) cudaStreamDestroy(aux2);
+  stream_release(aux, true, device);
+  stream_release(aux2, true, device);
 }
 
 cudaError_t FactorCtx::ensure(int nblk) {
-  if (!aux) {
-    int lo, hi;
-    CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-    CK(cudaStreamCreateWithPriority(&aux, cudaStreamNonBlocking, hi));
-  }
-  if (!aux2) {
-    int lo, hi;
-    CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-    CK(cudaStreamCreateWithPriority(&aux2, cudaStreamNonBlocking, hi));
-  }
+  if (!aux || !aux2) CK(cudaGetDevice(&device));
+  if (!aux) CK(stream_acquire(&aux, true));
+  if (!aux2) CK(stream_acquire(&aux2, true));
   for (auto& e : side)
     if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   while ((int)ev.size() < 3 * nblk + 2) {

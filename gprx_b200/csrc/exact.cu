@@ -26,7 +26,7 @@ ExactState::~ExactState() {
   if (stream) cudaStreamSynchronize(stream);
   for (auto& e : ev)
     if (e) cudaEventDestroy(e);
-  if (stream) cudaStreamDestroy(stream);
+  stream_release(stream, false, device);
 }
 
 static bool in_default_interval(double log_v) {
@@ -60,7 +60,7 @@ gprx_status ExactState::create(const double* xh, uint64_t nn, uint64_t dd, const
   ld = round_ld(cap);
   device = opt.device;
   GPRX_CUDA_TRY(cudaSetDevice(device));
-  GPRX_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  GPRX_CUDA_TRY(stream_acquire(&stream, false));
   for (auto& e : ev) GPRX_CUDA_TRY(cudaEventCreate(&e));
   int nblk = ceil_div(cap, NB);
   if (x.alloc((size_t)cap * d) != cudaSuccess || y.alloc(cap) != cudaSuccess ||

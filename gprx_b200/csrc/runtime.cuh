@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "pool.h"
 
 namespace gprx {
 
@@ -27,6 +28,7 @@ template <typename T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
+  int device = 0;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
@@ -34,7 +36,7 @@ struct DevBuf {
   cudaError_t alloc(size_t count) {
     reset();
     if (count == 0) return cudaSuccess;
-    cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
+    cudaError_t e = device_alloc((void**)&p, count * sizeof(T), &device);
     if (e != cudaSuccess) {
       p = nullptr;
       return e;
@@ -45,7 +47,7 @@ struct DevBuf {
   // grows (never shrinks); contents are not kept
   cudaError_t ensure(size_t count) { return count <= n ? cudaSuccess : alloc(count); }
   void reset() {
-    if (p) cudaFree(p);
+    device_free(p, n * sizeof(T), device);
     p = nullptr;
     n = 0;
   }
@@ -56,17 +58,18 @@ template <typename T>
 struct HostPinned {
   T* p = nullptr;
   size_t n = 0;
-  ~HostPinned() {
-    if (p) cudaFreeHost(p);
-  }
+  ~HostPinned() { reset(); }
   cudaError_t ensure(size_t count) {
     if (count <= n) return cudaSuccess;
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    n = 0;
-    cudaError_t e = cudaMallocHost((void**)&p, count * sizeof(T));
+    reset();
+    cudaError_t e = pinned_alloc((void**)&p, count * sizeof(T));
     if (e == cudaSuccess) n = count;
     return e;
+  }
+  void reset() {
+    pinned_free(p, n * sizeof(T));
+    p = nullptr;
+    n = 0;
   }
 };
 

@@ -351,7 +351,7 @@ struct SgprState {
     if (stream) cudaStreamSynchronize(stream);
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
-    if (stream) cudaStreamDestroy(stream);
+    stream_release(stream, false, device);
   }
 
   double noise() const { return std::exp(log_noise); }
@@ -472,7 +472,7 @@ gprx_status SgprState::create(const double* xh, uint64_t nn, uint64_t dd, const 
   ldm = round_ld(m);
   device = opt.device;
   GPRX_CUDA_TRY(cudaSetDevice(device));
-  GPRX_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  GPRX_CUDA_TRY(stream_acquire(&stream, false));
   for (auto& e : ev) GPRX_CUDA_TRY(cudaEventCreate(&e));
   int nblk = ceil_div(m, NB);
   // the m×m factors keep ld columns, the room a bordered inducing insert grows into
