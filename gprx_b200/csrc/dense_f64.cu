@@ -66,10 +66,10 @@ cudaError_t dgemm(bool ta, bool tb, const GemmParams& p, cudaStream_t s, int bat
 
 // B := A·B or Aᵀ·B in place (M, K ≤ 128): one tile holds every row of its
 // columns and reads them all before it writes.
-template <bool TA>
-static cudaError_t dgemm_inplace(const GemmParams& p, cudaStream_t s) {
+static cudaError_t dgemm_inplace(bool ta, const GemmParams& p, cudaStream_t s) {
   if (p.M > 128) return cudaErrorInvalidValue;
-  return launch_dgemm<128, 64, 32, 64, 16, 2, TA, false>(p, 1, s);
+  if (ta) return launch_dgemm<128, 64, 32, 64, 16, 2, true, false>(p, 1, s);
+  return launch_dgemm<128, 64, 32, 64, 16, 2, false, false>(p, 1, s);
 }
 
 GemmParams gemm_params(int M, int N, int K, const double* A, long long lda, const double* B, long long ldb,
@@ -667,75 +667,55 @@ cudaError_t lauum_lower(const double* X, long long ldx, int n, double* C, long l
   return dgemm_fill<true, false>(p, s, 1);
 }
 
-cudaError_t trsm_lower(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
-                       DevStatus* st, cudaStream_t s) {
-  if (tri_solve_few(n, q)) return tri_solve(L, ld, n, linv, B, ldb, q, false, st, s);
-  return trsm_lower_wide(L, ld, n, linv, B, ldb, q, st, s);
-}
-
-cudaError_t trsm_lower_wide(const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
-                            int q, DevStatus* st, cudaStream_t s) {
-  for (int k0 = 0; k0 < n; k0 += NB) {
-    int nbk = min(NB, n - k0);
-    const double* lk = linv + (long long)(k0 / NB) * NB * NB;
-    double* Bk = B + k0;
-    GemmParams p1 = gemm_params(nbk, q, nbk, lk, NB, Bk, ldb, Bk, ldb, 1.0, 0.0, st);
-    CK(dgemm_inplace<false>(p1, s));
-    int rest = n - k0 - nbk;
-    if (rest <= 0) break;
-    GemmParams p2 = gemm_params(rest, q, nbk, L + (k0 + nbk) + (long long)k0 * ld, ld, Bk, ldb, B + k0 + nbk, ldb,
-                                -1.0, 1.0, st);
-    CK(dgemm(false, false, p2, s));
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t trsm_lower_t(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
-                         DevStatus* st, cudaStream_t s) {
-  if (tri_solve_few(n, q)) return tri_solve(L, ld, n, linv, B, ldb, q, true, st, s);
-  int nblk = ceil_div(n, NB);
-  for (int kb = nblk - 1; kb >= 0; --kb) {
-    int k0 = kb * NB;
-    int nbk = min(NB, n - k0);
-    const double* lk = linv + (long long)kb * NB * NB;
-    double* Bk = B + k0;
-    // B_k := L_kk⁻ᵀ B_k
-    GemmParams p1 = gemm_params(nbk, q, nbk, lk, NB, Bk, ldb, Bk, ldb, 1.0, 0.0, st);
-    CK(dgemm_inplace<true>(p1, s));
-    if (k0 == 0) break;
-    // B_{<k} −= L_{k,<k}ᵀ B_k
-    GemmParams p2 = gemm_params(k0, q, nbk, L + k0, ld, Bk, ldb, B, ldb, -1.0, 1.0, st);
-    CK(dgemm(true, false, p2, s));
-  }
-  return cudaGetLastError();
-}
-
 // split point of a recursive solve: half of n rounded up to whole NB blocks
 // (the diagonal-block inverses are indexed by row / NB)
 static int rec_split(int n) { return ceil_div(ceil_div(n, 2), NB) * NB; }
 
-cudaError_t trsm_lower_rec(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
-                           int leaf, DevStatus* st, cudaStream_t s) {
-  const int n1 = rec_split(n);
-  if (n <= leaf || n1 >= n) return trsm_lower(L, ld, n, linv, B, ldb, q, st, s);
-  const int n2 = n - n1;
-  CK(trsm_lower_rec(L, ld, n1, linv, B, ldb, q, leaf, st, s));
-  GemmParams p = gemm_params(n2, q, n1, L + n1, ld, B, ldb, B + n1, ldb, -1.0, 1.0, st);
-  CK(dgemm(false, false, p, s));
-  return trsm_lower_rec(L + n1 + (long long)n1 * ld, ld, n2, linv + (long long)(n1 / NB) * NB * NB, B + n1, ldb, q,
-                        leaf, st, s);
+// The block a class's recursion ends with: one tri_solve launch up to so many
+// rows, or (SOLVE_BULK) one 128-row block times its inverse, in place.
+static int solve_leaf(int cls, int n) {
+  return cls == SOLVE_FEW ? n : cls == SOLVE_MID ? 512 : cls == SOLVE_WIDE ? 256 : NB;
+}
+static cudaError_t solve_block(int cls, const double* L, long long ld, int n, const double* linv, double* B,
+                               long long ldb, int q, bool trans, DevStatus* st, cudaStream_t s) {
+  if (cls != SOLVE_BULK) return tri_solve(L, ld, n, linv, B, ldb, q, trans, st, s);
+  return dgemm_inplace(trans, gemm_params(n, q, n, linv, NB, B, ldb, B, ldb, 1.0, 0.0, st), s);
 }
 
-cudaError_t trsm_lower_t_rec(const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
-                             int q, int leaf, DevStatus* st, cudaStream_t s) {
+cudaError_t trsm_lower(int cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+                       int q, DevStatus* st, cudaStream_t s) {
   const int n1 = rec_split(n);
-  if (n <= leaf || n1 >= n) return trsm_lower_t(L, ld, n, linv, B, ldb, q, st, s);
+  if (n <= solve_leaf(cls, n) || n1 >= n) return solve_block(cls, L, ld, n, linv, B, ldb, q, false, st, s);
   const int n2 = n - n1;
-  CK(trsm_lower_t_rec(L + n1 + (long long)n1 * ld, ld, n2, linv + (long long)(n1 / NB) * NB * NB, B + n1, ldb, q,
-                      leaf, st, s));
+  CK(trsm_lower(cls, L, ld, n1, linv, B, ldb, q, st, s));
+  GemmParams p = gemm_params(n2, q, n1, L + n1, ld, B, ldb, B + n1, ldb, -1.0, 1.0, st);
+  CK(dgemm(false, false, p, s));
+  return trsm_lower(cls, L + n1 + (long long)n1 * ld, ld, n2, linv + (long long)(n1 / NB) * NB * NB, B + n1, ldb, q,
+                    st, s);
+}
+
+cudaError_t trsm_lower_t(int cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+                         int q, DevStatus* st, cudaStream_t s) {
+  const int n1 = rec_split(n);
+  if (n <= solve_leaf(cls, n) || n1 >= n) return solve_block(cls, L, ld, n, linv, B, ldb, q, true, st, s);
+  const int n2 = n - n1;
+  CK(trsm_lower_t(cls, L + n1 + (long long)n1 * ld, ld, n2, linv + (long long)(n1 / NB) * NB * NB, B + n1, ldb, q, st,
+                  s));
   GemmParams p = gemm_params(n1, q, n2, L + n1, ld, B + n1, ldb, B, ldb, -1.0, 1.0, st);
   CK(dgemm(true, false, p, s));
-  return trsm_lower_t_rec(L, ld, n1, linv, B, ldb, q, leaf, st, s);
+  return trsm_lower_t(cls, L, ld, n1, linv, B, ldb, q, st, s);
+}
+
+cudaError_t trsm_lower(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
+                       DevStatus* st, cudaStream_t s) {
+  if (q == 1) return tri_solve_vec(L, ld, n, linv, B, false, st, s);
+  return trsm_lower(solve_class(n, q), L, ld, n, linv, B, ldb, q, st, s);
+}
+
+cudaError_t trsm_lower_t(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
+                         DevStatus* st, cudaStream_t s) {
+  if (q == 1) return tri_solve_vec(L, ld, n, linv, B, true, st, s);
+  return trsm_lower_t(solve_class(n, q), L, ld, n, linv, B, ldb, q, st, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -60,34 +60,33 @@ cudaError_t lauum_lower(const double* X, long long ldx, int n, double* C, long l
 
 struct EmuWork;
 
-// B (n×q, ldb) := L⁻¹ B   /   := L⁻ᵀ B, with L's diagonal block inverses:
-// tri_solve where tri_solve_few says so, else (trsm_lower_wide) two GEMMs per
-// 128 rows.
+// B (n×q, ldb) := L⁻¹ B   /   := L⁻ᵀ B, with L's diagonal block inverses: by
+// recursive halving (X1 from the top half, one update B2 −= L21 X1 with K = n/2,
+// then the bottom half; the transpose bottom half first) down to blocks that
+// tri_solve takes in one launch (SOLVE_BULK: to 128-row blocks).  The class (solve_class of the whole solve)
+// fixes where the recursion stops, and with it the bits of a column: they do
+// not depend on q within a class.
+enum SolveClass : int { SOLVE_FEW = 0, SOLVE_MID = 1, SOLVE_WIDE = 2, SOLVE_BULK = 3 };
+int solve_class(long long n, long long q);
 cudaError_t trsm_lower(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
                        DevStatus* st, cudaStream_t s);
 cudaError_t trsm_lower_t(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
                          DevStatus* st, cudaStream_t s);
+cudaError_t trsm_lower(int cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+                       int q, DevStatus* st, cudaStream_t s);
+cudaError_t trsm_lower_t(int cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+                         int q, DevStatus* st, cudaStream_t s);
 
-cudaError_t trsm_lower_wide(const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
-                            int q, DevStatus* st, cudaStream_t s);
-
-// The same two solves (trans: L⁻ᵀ) with few right-hand sides in one launch of
-// thread-block clusters (tri_solve.cu); a column's bits do not depend on q.
-// prefix (one right-hand side): prefix[i + s·ldp] receives the sum of L(i, :)
-// x over the columns of the first s + 1 blocks, for the rows below block s.
-bool tri_solve_few(long long n, long long q);
+// The same two solves (trans: L⁻ᵀ) in one launch of thread-block clusters
+// (tri_solve.cu); a column's bits do not depend on q.  Any q for n ≤ 8192,
+// one right-hand side for every n.
 cudaError_t tri_solve(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
-                      bool trans, const DevStatus* st, cudaStream_t s, double* prefix = nullptr, long long ldp = 0);
-
-// The same two solves for wide B (q ≫ n) by recursive halving: X1 from the
-// top half, one rank-n1 update B2 −= L21 X1 (L21ᵀ X2 for the transpose), then
-// the bottom half; blocks of at most `leaf` rows use trsm_lower /
-// trsm_lower_t.  The updates have K = n/2, n/4, … instead of NB, so the
-// DGEMMs run near their large-K rate.
-cudaError_t trsm_lower_rec(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
-                           int leaf, DevStatus* st, cudaStream_t s);
-cudaError_t trsm_lower_t_rec(const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
-                             int q, int leaf, DevStatus* st, cudaStream_t s);
+                      bool trans, const DevStatus* st, cudaStream_t s);
+// One right-hand side in FP64 FMAs (other bits than tri_solve's).  prefix
+// (forward only): prefix[i + s·ldp] receives the sum of L(i, :) x over the
+// columns of the first s + 1 blocks, for the rows below block s.
+cudaError_t tri_solve_vec(const double* L, long long ld, int n, const double* linv, double* b, bool trans,
+                          const DevStatus* st, cudaStream_t s, double* prefix = nullptr, long long ldp = 0);
 
 // out = log|det L|² contribution: 2 Σ ln L_ii (lower LLT) or Σ ln D_i (ldlt=true).
 cudaError_t logdet_diag(const double* L, long long ld, int n, bool ldlt, double* out, DevStatus* st,

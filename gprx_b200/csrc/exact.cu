@@ -845,7 +845,7 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
   GPRX_CUDA_TRY(pred_h.ensure(2 * (size_t)qc_max));
   double* const hm = pred_h.p;
   // one route for the whole call: a query's bits do not depend on its chunk
-  const bool few = tri_solve_few(n, (long long)q);
+  const int cls = solve_class(n, (long long)q);
   const double kss = kern.diag_value();
   for (uint64_t c0 = 0; c0 < q; c0 += qc_max) {
     int qc = (int)std::min<uint64_t>(qc_max, q - c0);
@@ -857,8 +857,7 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
                                     cudaMemcpyHostToDevice, stream));
     GPRX_CUDA_TRY(fill_cross(kern, x.p, cap, n, xq, qc, qc, qbuf.p, ld, status.p, stream));
     GPRX_CUDA_TRY(gemv_t(qbuf.p, ld, n, qc, false, alpha.p, mdev, status.p, stream));
-    if (few) GPRX_CUDA_TRY(tri_solve(A.p, ld, n, linv.p, qbuf.p, ld, qc, false, status.p, stream));
-    else GPRX_CUDA_TRY(trsm_lower_wide(A.p, ld, n, linv.p, qbuf.p, ld, qc, status.p, stream));
+    GPRX_CUDA_TRY(trsm_lower(cls, A.p, ld, n, linv.p, qbuf.p, ld, qc, status.p, stream));
     GPRX_CUDA_TRY(col_sumsq(qbuf.p, ld, n, qc, online ? tmpv.p : nullptr, quad, status.p, stream));
     finish_var_kernel<<<ceil_div(qc, 256), 256, 0, stream>>>(quad, qc, kss, noise(), kind, vdev, status.p);
     count_launch();

@@ -295,8 +295,8 @@ gprx_status ExactState::online_delete(uint64_t id) {
     if (lead > 0) GPRX_CUDA_TRY(cudaMemsetAsync(p, 0, sizeof(double) * lead, stream));
     GPRX_CUDA_TRY(cudaMemcpyAsync(p + lead, A.p + (idx + 1) + (long long)idx * ld, sizeof(double) * (n - idx - 1),
                                   cudaMemcpyDeviceToDevice, stream));
-    GPRX_CUDA_TRY(tri_solve(A.p + row0 + (long long)row0 * ld, ld, len, linv.p + (long long)(row0 / NB) * NB * NB, p,
-                            len, 1, false, status.p, stream, prefix, len));
+    GPRX_CUDA_TRY(tri_solve_vec(A.p + row0 + (long long)row0 * ld, ld, len, linv.p + (long long)(row0 / NB) * NB * NB,
+                                p, false, status.p, stream, prefix, len));
     GPRX_LAUNCH(ldlt_rank1_scan_kernel, 1, R1_THREADS, 0, stream, A.p, ld, row0, idx + 1, n, idx, p, beta, dnew,
                 status.p);
   }

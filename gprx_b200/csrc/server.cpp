@@ -47,7 +47,7 @@
 #include "../../include/gprx_cuda.h"
 
 namespace gprx {
-bool tri_solve_few(long long n, long long q);  // dense_f64.cuh
+int solve_class(long long n, long long q);  // dense_f64.cuh
 }
 
 namespace {
@@ -275,13 +275,14 @@ uint64_t gprx_server::pick(std::vector<uint64_t>& batch) {
   } else if (head->kind == PREDICT) {
     // consecutive predicts of the same kind share one launch, as long as the
     // merged call solves the way each would alone (the same bits either way)
-    const bool few = gprx::tri_solve_few((long long)m.n, (long long)head->q);
+    const int cls = gprx::solve_class((long long)m.n, (long long)head->q);
     uint64_t total = head->q;
     while (!m.queue.empty()) {
       Request* nx = reqs[m.queue.front()].get();
       if (nx->kind != PREDICT || nx->vkind != head->vkind || small_predict(nx)) break;
-      if (gprx::tri_solve_few((long long)m.n, (long long)nx->q) != few) break;
-      if (few && !gprx::tri_solve_few((long long)m.n, (long long)(total + nx->q))) break;
+      if (gprx::solve_class((long long)m.n, (long long)nx->q) != cls ||
+          gprx::solve_class((long long)m.n, (long long)(total + nx->q)) != cls)
+        break;
       total += nx->q;
       batch.push_back(nx->id);
       m.queue.pop_front();

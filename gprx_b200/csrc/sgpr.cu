@@ -330,7 +330,6 @@ struct SgprState {
   static constexpr int EMU_S = 7;                // int8 digits per entry
   static constexpr int EMU_PART_K = 32768;       // K of one split-K part: K·S·2^12 < 2^31 keeps its int32 sums exact
   static constexpr int EMU_GROUP = 8 * EMU_PART_K;  // columns of n sliced at a time (8 parts in flight)
-  static constexpr int TRSM_LEAF = 256;          // rows of the blocked solves under the recursive m×n solves
   bool use_emu() const { return opt.precision == GPRX_PRECISION_MIXED && n >= EMU_MIN_N; }
   gprx_status ensure_emu(EmuWork& w);
   HostPinned<double> res_h;
@@ -655,7 +654,7 @@ gprx_status SgprState::assemble() {
     if ((st = ensure_emu(ew)) != GPRX_OK) return st;
     GPRX_CUDA_TRY(cudaMemsetAsync(emu_err.p, 0, sizeof(int), stream));
   }
-  GPRX_CUDA_TRY(trsm_lower_rec(Lmm.p, ldm, m, linv_mm.p, Amat.p, ldm, nn, TRSM_LEAF, status.p, stream));
+  GPRX_CUDA_TRY(trsm_lower(Lmm.p, ldm, m, linv_mm.p, Amat.p, ldm, nn, status.p, stream));
   GPRX_CUDA_TRY(cudaEventRecord(ev[1], stream));
   // B = A Aᵀ + σ² I, L_B
   if (emu) {
@@ -738,8 +737,8 @@ gprx_status SgprState::gradient(double* grad) {
     GPRX_CUDA_TRY(cudaMemsetAsync(emu_err.p, 0, sizeof(int), stream));
   }
   GPRX_CUDA_TRY(cudaMemcpyAsync(G.p, Amat.p, sizeof(double) * ldm * nn, cudaMemcpyDeviceToDevice, stream));
-  GPRX_CUDA_TRY(trsm_lower_rec(Bl.p, ldm, m, linv_B.p, G.p, ldm, nn, TRSM_LEAF, status.p, stream));
-  GPRX_CUDA_TRY(trsm_lower_t_rec(Bl.p, ldm, m, linv_B.p, G.p, ldm, nn, TRSM_LEAF, status.p, stream));
+  GPRX_CUDA_TRY(trsm_lower(Bl.p, ldm, m, linv_B.p, G.p, ldm, nn, status.p, stream));
+  GPRX_CUDA_TRY(trsm_lower_t(Bl.p, ldm, m, linv_B.p, G.p, ldm, nn, status.p, stream));
   adjoint_update_kernel<<<grid_for((long long)nn * 32, 256), 256, 0, stream>>>(Amat.p, G.p, ldm, m, nn, w.p, y.p,
                                                                                 1.0 / noise_v, status.p);
   count_launch();
@@ -750,7 +749,7 @@ gprx_status SgprState::gradient(double* grad) {
   } else {
     GPRX_CUDA_TRY(syrk_splitk(G.p, ldm, m, nn, Amat.p, ldm, false, 0.0, splitbuf, H.p, ldm, status.p, stream));
   }
-  GPRX_CUDA_TRY(trsm_lower_t_rec(Lmm.p, ldm, m, linv_mm.p, G.p, ldm, nn, TRSM_LEAF, status.p, stream));
+  GPRX_CUDA_TRY(trsm_lower_t(Lmm.p, ldm, m, linv_mm.p, G.p, ldm, nn, status.p, stream));
   // w_mm = −sym(L⁻ᵀ tril½(H) L⁻¹)
   tril_half_kernel<<<grid_for((long long)m * m, 256), 256, 0, stream>>>(H.p, ldm, m, Xb.p);
   count_launch();
@@ -1293,7 +1292,7 @@ gprx_status SgprState::factor_kmm_and_a(EmuWork& ew, bool& emu) {
     if ((st = ensure_emu(ew)) != GPRX_OK) return st;
     GPRX_CUDA_TRY(cudaMemsetAsync(emu_err.p, 0, sizeof(int), stream));
   }
-  GPRX_CUDA_TRY(trsm_lower_rec(Lmm.p, ldm, m, linv_mm.p, Amat.p, ldm, nn, TRSM_LEAF, status.p, stream));
+  GPRX_CUDA_TRY(trsm_lower(Lmm.p, ldm, m, linv_mm.p, Amat.p, ldm, nn, status.p, stream));
   return GPRX_OK;
 }
 
@@ -1387,8 +1386,8 @@ gprx_status SgprState::shard_nlml(const double* e1, double* nlml_out, double* e2
     GPRX_CUDA_TRY(cudaMemsetAsync(emu_err.p, 0, sizeof(int), stream));
   }
   GPRX_CUDA_TRY(cudaMemcpyAsync(G.p, Amat.p, sizeof(double) * ldm * nn, cudaMemcpyDeviceToDevice, stream));
-  GPRX_CUDA_TRY(trsm_lower_rec(Bl.p, ldm, m, linv_B.p, G.p, ldm, nn, TRSM_LEAF, status.p, stream));
-  GPRX_CUDA_TRY(trsm_lower_t_rec(Bl.p, ldm, m, linv_B.p, G.p, ldm, nn, TRSM_LEAF, status.p, stream));
+  GPRX_CUDA_TRY(trsm_lower(Bl.p, ldm, m, linv_B.p, G.p, ldm, nn, status.p, stream));
+  GPRX_CUDA_TRY(trsm_lower_t(Bl.p, ldm, m, linv_B.p, G.p, ldm, nn, status.p, stream));
   adjoint_update_kernel<<<grid_for((long long)nn * 32, 256), 256, 0, stream>>>(Amat.p, G.p, ldm, m, nn, w.p, y.p,
                                                                                 1.0 / noise_v, status.p);
   count_launch();
@@ -1398,7 +1397,7 @@ gprx_status SgprState::shard_nlml(const double* e1, double* nlml_out, double* e2
   } else {
     GPRX_CUDA_TRY(syrk_splitk(G.p, ldm, m, nn, Amat.p, ldm, false, 0.0, splitbuf, e2, m, status.p, stream));
   }
-  GPRX_CUDA_TRY(trsm_lower_t_rec(Lmm.p, ldm, m, linv_mm.p, G.p, ldm, nn, TRSM_LEAF, status.p, stream));
+  GPRX_CUDA_TRY(trsm_lower_t(Lmm.p, ldm, m, linv_mm.p, G.p, ldm, nn, status.p, stream));
   int b2 = 0;
   GPRX_CUDA_TRY(cross_contract(kern, z.p, m, m, x.p, cap, nn, G.p, ldm, partials.p, &b2, status.p, stream));
   GPRX_CUDA_TRY(grad_finalize(kern, partials.p, b2, slot_param.p, 1.0, 0.0, e2 + mm2, status.p, stream));

@@ -42,8 +42,6 @@ struct TriSolveArgs {
   long long ldb;
   int q;
   int C;
-  double* prefix;
-  long long ldp;
   const DevStatus* st;
 };
 
@@ -161,7 +159,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(TriSolveArgs g
   };
   // sums of owned block index o += (tile at i0, k0) · x; from shared memory
   // when staged, else from global in batches of eight k steps, one ahead.
-  auto fold = [&](int o, int i0, int k0, int s, bool staged) {
+  auto fold = [&](int o, int i0, int k0, bool staged) {
     double a[NT][2][4];
 #pragma unroll
     for (int t = 0; t < NT; ++t)
@@ -208,10 +206,6 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(TriSolveArgs g
     for (int t = 0; t < NT; ++t)
 #pragma unroll
       for (int r = 0; r < 4; ++r) set_sum(o, t, r, a[t][0][r] + a[t][1][r]);
-    if (NT == 1 && g.prefix && t4 == 0)
-#pragma unroll
-      for (int r = 0; r < 4; r += 2)
-        if (i0 + r0 + 4 * r < n) g.prefix[(i0 + r0 + 4 * r) + s * g.ldp] = a[0][0][r] + a[0][1][r];
   };
 
   if (rank == 0) {
@@ -232,11 +226,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(TriSolveArgs g
     if (mine) cp_async_wait<0>();
     __syncthreads();
     if (mine) {
-      fold((s + 1) / C, first(s + 1), k0, s, true);
+      fold((s + 1) / C, first(s + 1), k0, true);
       solve(s + 1);
     }
     cluster_arrive();
-    for (int t = s + 2 + (rank - (s + 2) % C + C) % C; t < nblk; t += C) fold(t / C, first(t), k0, s, false);
+    for (int t = s + 2 + (rank - (s + 2) % C + C) % C; t < nblk; t += C) fold(t / C, first(t), k0, false);
     if ((s + 2) % C == rank && s + 2 < nblk) {
       if (C == 1) __syncthreads();  // this CTA also used the tile at this step
       prefetch(s + 2);
@@ -245,15 +239,190 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(TriSolveArgs g
   }
 }
 
-template <bool TRANS, int NT>
-cudaError_t ts_launch(const TriSolveArgs& g, int strips, size_t smem, cudaStream_t s) {
-  auto kern = tri_solve_kernel<TRANS, NT>;
+// ---------------------------------------------------------------------------
+// one right-hand side that is a vector of its own (α, the online updates)
+// ---------------------------------------------------------------------------
+// The same steps on FP64 FMAs: a DMMA spends seven eighths of its columns on
+// one right-hand side (2 K cycles a 128×128 tile, 16 FMA a cycle and scheduler
+// either way), here a tile costs 64 FMAs a thread.  L_{s+1,s} waits in
+// registers, the diagonal block's inverse in shared memory.  Forward, a thread
+// owns a row and half of the k range (column-major L: coalesced over rows);
+// transposed, a warp owns 16 rows of Lᵀ, its lanes run along k, and a
+// reduce-scatter of 16 shuffles leaves row ii in lanes 2·ii, 2·ii + 1.
+// Measured (forward / transposed, µs, DMMA → FMA): n = 512 23 / 23 → 18 / 18,
+// n = 2000 83 / 83 → 59 / 55, n = 4096 229 / 201 → 151 / 127.
+struct TriVecArgs {
+  const double* L;
+  long long ld;
+  int n;
+  const double* linv;
+  double* b;
+  int C;
+  double* prefix;
+  long long ldp;
+  const DevStatus* st;
+};
+
+inline size_t tv_smem(int own) { return sizeof(double) * ((size_t)NB * NB + 4 * NB + (size_t)own * NB); }
+
+// v[ii] of 32 lanes summed; lane l returns row l / 2.
+__device__ __forceinline__ double scatter16(double (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int m = 8; m >= 1; m /= 2) {
+    const bool up = lane & (2 * m);
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      const double send = up ? v[i] : v[i + m], keep = up ? v[i + m] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * m);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+template <bool TRANS>
+__global__ void __launch_bounds__(TS_THREADS, 1) tri_vec_kernel(TriVecArgs g) {
+  extern __shared__ __align__(16) double ts_sm[];
+  if (dev_failed(g.st)) return;  // the same word for the whole cluster
+  double* li = ts_sm;           // the owned diagonal block's inverse, ld NB
+  double* xs = li + NB * NB;    // x_s
+  double* bs = xs + NB;         // right-hand side of the owned block
+  double* part = bs + NB;       // [half][row]
+  double* sums = part + 2 * NB;  // [owned block][row]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n = g.n, C = g.C, rank = blockIdx.x % C, nblk = (n + NB - 1) / NB;
+  const int row = tid & (NB - 1), half = tid >> 7, kb = 64 * half;  // forward
+  auto first = [&](int s) { return (TRANS ? nblk - 1 - s : s) * NB; };
+  const int own = (nblk - rank + C - 1) / C;
+  for (int e = tid; e < own * NB; e += TS_THREADS) sums[e] = 0.0;
+  double f[64];
+  auto load_tile = [&](int i0, int k0) {
+#pragma unroll
+    for (int u = 0; u < 64; ++u) {
+      if (TRANS) {
+        const int k = k0 + lane + 32 * (u & 3);
+        f[u] = k < n ? g.L[k + (long long)(i0 + 16 * warp + (u >> 2)) * g.ld] : 0.0;
+      } else {
+        f[u] = i0 + row < n ? g.L[(i0 + row) + (long long)(k0 + kb + u) * g.ld] : 0.0;
+      }
+    }
+  };
+  auto prefetch = [&](int s) {
+    const double* src = g.linv + (long long)(first(s) / NB) * NB * NB;
+    for (int e = 2 * tid; e < NB * NB; e += 2 * TS_THREADS) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(li + e);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + e));
+    }
+    cp_async_commit();
+    if (s > 0) load_tile(first(s), first(s - 1));
+  };
+  // (tile in f) · x into the sums of owned block o
+  auto fold = [&](int o, int i0, int s) {
+    if (TRANS) {
+      double v[16], x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = xs[lane + 32 * u];
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        v[i] = fma(f[4 * i], x[0], f[4 * i + 1] * x[1]) + fma(f[4 * i + 2], x[2], f[4 * i + 3] * x[3]);
+      const double t = scatter16(v);
+      if (!(lane & 1)) sums[o * NB + 16 * warp + (lane >> 1)] += t;
+    } else {
+      double a[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int u = 0; u < 64; u += 2) {
+        const double2 x = *reinterpret_cast<const double2*>(xs + kb + u);
+        a[u & 2] = fma(f[u], x.x, a[u & 2]);
+        a[(u & 2) + 1] = fma(f[u + 1], x.y, a[(u & 2) + 1]);
+      }
+      __syncthreads();  // the previous fold's reads of part are done
+      part[tid] = (a[0] + a[1]) + (a[2] + a[3]);
+      __syncthreads();
+      if (tid < NB) {
+        const double t = sums[o * NB + tid] + (part[tid] + part[NB + tid]);
+        sums[o * NB + tid] = t;
+        if (g.prefix && i0 + tid < n) g.prefix[(i0 + tid) + s * g.ldp] = t;
+      }
+    }
+  };
+  auto solve = [&](int s) {
+    const int i0 = first(s), o = s / C;
+    cp_async_wait<0>();
+    __syncthreads();
+    if (tid < NB) bs[tid] = i0 + tid < n ? g.b[i0 + tid] - sums[o * NB + tid] : 0.0;
+    __syncthreads();
+    if (TRANS) {  // Σ_{k ≥ i} X(k, i) b_k
+      double v[16], x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = bs[lane + 32 * u];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        v[i] = 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (32 * u + 31 >= 16 * warp) v[i] = fma(li[(16 * warp + i) * NB + lane + 32 * u], x[u], v[i]);
+      }
+      const double t = scatter16(v);
+      const int i = i0 + 16 * warp + (lane >> 1);
+      if (!(lane & 1) && i < n) g.b[i] = t;
+    } else {  // Σ_{k ≤ i} X(i, k) b_k
+      double a[4] = {0, 0, 0, 0};
+      const int end = min(64, (row | 31) + 1 - kb);
+#pragma unroll 8
+      for (int u = 0; u < end; u += 4) {
+        const double2 x0 = *reinterpret_cast<const double2*>(bs + kb + u);
+        const double2 x1 = *reinterpret_cast<const double2*>(bs + kb + u + 2);
+        a[0] = fma(li[(kb + u) * NB + row], x0.x, a[0]);
+        a[1] = fma(li[(kb + u + 1) * NB + row], x0.y, a[1]);
+        a[2] = fma(li[(kb + u + 2) * NB + row], x1.x, a[2]);
+        a[3] = fma(li[(kb + u + 3) * NB + row], x1.y, a[3]);
+      }
+      part[tid] = (a[0] + a[1]) + (a[2] + a[3]);
+      __syncthreads();
+      if (tid < NB && i0 + tid < n) g.b[i0 + tid] = part[tid] + part[NB + tid];
+    }
+  };
+
+  if (rank == 0) {
+    prefetch(0);
+    solve(0);
+  }
+  cluster_arrive();
+  if (rank == 1 % C && nblk > 1) {
+    __syncthreads();
+    prefetch(1);
+  }
+  cluster_wait();
+  for (int s = 0; s + 1 < nblk; ++s) {
+    const int k0 = first(s);
+    __syncthreads();  // the previous step's reads of xs are done
+    if (tid < NB) xs[tid] = k0 + tid < n ? __ldcg(g.b + k0 + tid) : 0.0;
+    __syncthreads();
+    if ((s + 1) % C == rank) {
+      fold((s + 1) / C, first(s + 1), s);
+      solve(s + 1);
+    }
+    cluster_arrive();
+    for (int t = s + 2 + (rank - (s + 2) % C + C) % C; t < nblk; t += C) {
+      load_tile(first(t), k0);
+      fold(t / C, first(t), s);
+    }
+    if ((s + 2) % C == rank && s + 2 < nblk) {
+      if (C == 1) __syncthreads();  // this CTA also used the inverse at this step
+      prefetch(s + 2);
+    }
+    cluster_wait();
+  }
+}
+
+template <typename Args>
+cudaError_t ts_launch(void (*kern)(Args), const Args& g, int ctas, size_t smem, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX);
   if (e != cudaSuccess) return e;
   if (g.C > 8 && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
     return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(strips * g.C));
+  cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(TS_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -316,26 +485,45 @@ bool ts_plan(int n, int q, int* NT, int* C) {
 
 }  // namespace
 
-// Few right-hand sides: n·q ≤ 3·2²⁰.  Measured against trsm_lower_wide (µs):
-// n = 512: q = 256 33 / 205, 4000 128 / 211, 10000 285 / 268; n = 1000:
-// q = 256 117 / 435, 2000 253 / 443, 4000 501 / 529; n = 2000: q = 1 80 / 851,
-// 256 263 / 894, 1000 644 / 898, 2000 1162 / 1080; n = 4096: q = 1 193 / 1747,
-// 500 1574 / 1871, 1000 2850 / 2235.
-bool tri_solve_few(long long n, long long q) {
+// One launch while the strips' reads of L are small: n·q ≤ 200 000, and one
+// right-hand side always.  Above, recursion with blocks of 512 rows up to
+// q = 1200 and of 256 rows from there on.  Measured (µs, one launch / 512 / 256 /
+// two GEMMs per 128 rows): n = 512, q = 500 37 / 37 / 45 / 94; n = 1000, q = 64
+// 61 / 83 / 108 / 193, 256 119 / 83 / 108 / 192, 1000 130 / 104 / 122 / 232, 2000
+// 255 / 192 / 176 / 281; n = 4096, q = 1 193 / – / – / 807, 64 328 / 478 / 579 /
+// 807, 256 1005 / 551 / 636 / 1011, 1500 – / 1627 / 1546 / 1881, 10000 – / 6887 /
+// 6785 / 7763.  From q = 16384 on the launch's L2 reads (n²/2 values for every
+// 16 columns) cost more than products of 128-row blocks with their inverses: an
+// Sgpr evaluation (m = 1024, q = 10⁶) takes 344 ms with blocks of 256, 307 ms so.
+int solve_class(long long n, long long q) {
   int nt, c;
-  return n > 0 && q > 0 && n * q <= (3LL << 20) && ts_plan((int)n, (int)q, &nt, &c);
+  if (q == 1 || (n * q <= 200000 && ts_plan((int)n, (int)q, &nt, &c))) return SOLVE_FEW;
+  return q <= 1200 ? SOLVE_MID : q <= 16384 ? SOLVE_WIDE : SOLVE_BULK;
 }
 
 cudaError_t tri_solve(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
-                      bool trans, const DevStatus* st, cudaStream_t s, double* prefix, long long ldp) {
+                      bool trans, const DevStatus* st, cudaStream_t s) {
   if (n <= 0 || q <= 0) return cudaSuccess;
   int nt, c;
-  if (!ts_plan(n, q, &nt, &c) || (prefix && q != 1)) return cudaErrorInvalidValue;
-  TriSolveArgs g{L, ld, n, linv, B, ldb, q, c, prefix, ldp, st};
+  if (!ts_plan(n, q, &nt, &c)) return cudaErrorInvalidValue;
+  const TriSolveArgs g{L, ld, n, linv, B, ldb, q, c, st};
   const int strips = ceil_div(q, 8 * nt);
   const size_t smem = ts_smem(nt, ceil_div(ceil_div(n, NB), c), q == 1);
-  if (trans) return nt == 1 ? ts_launch<true, 1>(g, strips, smem, s) : ts_launch<true, 2>(g, strips, smem, s);
-  return nt == 1 ? ts_launch<false, 1>(g, strips, smem, s) : ts_launch<false, 2>(g, strips, smem, s);
+  void (*kern)(TriSolveArgs) = trans ? (nt == 1 ? tri_solve_kernel<true, 1> : tri_solve_kernel<true, 2>)
+                                     : (nt == 1 ? tri_solve_kernel<false, 1> : tri_solve_kernel<false, 2>);
+  return ts_launch(kern, g, strips * c, smem, s);
+}
+
+cudaError_t tri_solve_vec(const double* L, long long ld, int n, const double* linv, double* b, bool trans,
+                          const DevStatus* st, cudaStream_t s, double* prefix, long long ldp) {
+  if (n <= 0) return cudaSuccess;
+  const int nblk = ceil_div(n, NB), cmax = ts_cluster16() ? TS_MAX_CLUSTER : 8;
+  int c = 1;
+  while (c * 2 <= cmax && c * 2 <= nblk) c *= 2;
+  const size_t smem = tv_smem(ceil_div(nblk, c));
+  if (smem > TS_SMEM_MAX || (prefix && trans)) return cudaErrorInvalidValue;
+  const TriVecArgs g{L, ld, n, linv, b, c, prefix, ldp, st};
+  return ts_launch(trans ? tri_vec_kernel<true> : tri_vec_kernel<false>, g, c, smem, s);
 }
 
 }  // namespace gprx
