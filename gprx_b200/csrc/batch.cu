@@ -341,6 +341,171 @@ __device__ void cta_trtri(const Work& w, int n, long long ld, double* smem, int 
   __syncthreads();
 }
 
+// A problem of at most one diagonal block, held in shared memory from the fill
+// to the gradient: K, L and X = L⁻¹ (diag_block.cuh's layout), then K⁻¹ = XᵀX
+// over L.  Nothing but x, y and the results touches global memory.  α goes to
+// `alpha` (n values), the gradient's slot sums to `slots`; *logdet and *quad are
+// set in every thread.  Returns −1, the failing column, or SMALL_NONFINITE.
+constexpr int SMALL_NONFINITE = -2;
+inline size_t tile_smem() {
+  return (size_t)(2 * GPRX_MAX_DIM * FT_B + 2 * FT_B + (BT / 32) * 64) * sizeof(double);
+}
+inline size_t small_smem() { return diag_block_smem() + tile_smem() + 2 * NB_DIAG * sizeof(double); }
+
+template <int ARD_D>
+__device__ int cta_small(const KTree& tree, const double* x, const double* y, int n, double diag_add, double* smem,
+                         int* flag_sh, double* red, double* slots, double* alpha, double* logdet, double* quad) {
+  double* s = smem;
+  double* tmp = s + NB_DIAG * FLS;
+  double* ldiag = tmp + TMP_DOUBLES + NB_DIAG;
+  double* z = ldiag + NB_DIAG;  // then α, then the tiles' scratch
+  double* av = z + NB_DIAG;
+  double* tiles = av + NB_DIAG;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int np = (n + LF - 1) / LF, npad = np * LF;
+  if (!cta_fill_any<ARD_D>(tree, x, n, s, FLS, diag_add, tiles, flag_sh)) return SMALL_NONFINITE;
+  diag_block_pad(s, n);
+  const int f = diag_block_core(nullptr, 0, 0, n, nullptr, false, smem, flag_sh);
+  if (f >= 0) return f;
+  double acc = 0.0;
+  for (int i = tid; i < n; i += BT) acc += log(ldiag[i]);
+  *logdet = 2.0 * block_sum(acc, red);
+  // z = X y, α = Xᵀ z; X(i, j) is s[j + i·FLS]
+  for (int i = warp; i < n; i += BT / 32) {
+    double v = 0.0;
+    for (int j = lane; j <= i; j += 32) v = fma(s[j + i * FLS], y[j], v);
+    v = warp_sum(v);
+    if (lane == 0) z[i] = v;
+  }
+  __syncthreads();
+  {
+    const int j = tid & (NB_DIAG - 1), part = tid / NB_DIAG;
+    double v = 0.0;
+    for (int i = j + part; i < n; i += BT / NB_DIAG) v = fma(s[j + i * FLS], z[i], v);
+    tmp[tid] = v;
+  }
+  __syncthreads();
+  if (tid < n) {
+    double v = 0.0;
+#pragma unroll
+    for (int part = 0; part < BT / NB_DIAG; ++part) v += tmp[part * NB_DIAG + tid];
+    av[tid] = v;
+    alpha[tid] = v;
+  }
+  __syncthreads();
+  acc = 0.0;
+  for (int i = tid; i < n; i += BT) acc = fma(y[i], av[i], acc);
+  *quad = block_sum(acc, red);
+  // K⁻¹(i, j) = Σ_{k ≥ i} X(k, i) X(k, j): 16×16 lower tiles (36 at most) in
+  // registers, written over L once every warp has read X
+  constexpr int KT = (NB_DIAG / LF * (NB_DIAG / LF + 1) / 2 + BT / 32 - 1) / (BT / 32);
+  double c[KT][2][4];
+#pragma unroll
+  for (int u = 0; u < KT; ++u) {
+    const int t = warp + u * (BT / 32);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) c[u][h][r] = 0.0;
+    if (t >= np * (np + 1) / 2) continue;
+    int ti = 0;
+    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+    const int i0 = LF * ti, j0 = LF * (t - ti * (ti + 1) / 2);
+#pragma unroll 2
+    for (int kk = i0; kk < npad; kk += 4) {
+      const int k = kk + t4;
+      const double* col = s + k * FLS;
+      const double a0 = k >= i0 + g ? col[i0 + g] : 0.0, a1 = k >= i0 + g + 8 ? col[i0 + g + 8] : 0.0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = j0 + 8 * h + g;
+        dmma_16x8x4(c[u][h], a0, a1, k >= j ? col[j] : 0.0);
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < KT; ++u) {
+    const int t = warp + u * (BT / 32);
+    if (t >= np * (np + 1) / 2) continue;
+    int ti = 0;
+    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+    const int i0 = LF * ti, j0 = LF * (t - ti * (ti + 1) / 2);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row = i0 + g + ((r & 2) ? 8 : 0), col = j0 + 8 * h + 2 * t4 + (r & 1);
+        if (row >= col) s[row + col * FLS] = c[u][h][r];
+      }
+  }
+  __syncthreads();
+  cta_grad_any<ARD_D>(tree, x, n, s, FLS, av, tiles, slots);
+  return -1;
+}
+
+// θ gradient of −½⟨W, ∂K/∂θ⟩ from the slot sums (one thread).
+__device__ inline void slots_to_grad(const double* slots, int ns, const int* slot_param, double noise, int p,
+                                     double* g) {
+  for (int i = 0; i < p; ++i) g[i] = 0.0;
+  for (int s = 0; s < ns - 1; ++s) {
+    const int pi = slot_param[s];
+    if (pi >= 0) g[pi] += slots[s];
+  }
+  for (int i = 0; i < p - 1; ++i) g[i] *= -0.5;
+  g[p - 1] = -0.5 * noise * slots[ns - 1];
+}
+
+// One evaluation of one exact problem of at most 128 points in one launch: the
+// log-det, yᵀα and the gradient to res[0], res[1], res[2 ..], α to alpha.
+// Latency-bound: the pivots' chain and a few passes over one block.  As 12
+// launches (fill, diagonal step, log-det, copy, two products, two vector
+// products, a dot product, K⁻¹, gradient, its sums) n = 64 took 108 µs.
+template <int ARD_D>
+__global__ void __launch_bounds__(BT, 1) small_eval_kernel(const __grid_constant__ KTree tree, const double* x,
+                                                           const double* y, int n, double diag_add, double noise,
+                                                           int p, const int* slot_param, double* alpha, double* res,
+                                                           DevStatus* st) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ int flag_sh;
+  __shared__ double red[32];
+  __shared__ double slots[64];
+  if (dev_failed(st)) return;
+  double logdet, quad;
+  const int f = cta_small<ARD_D>(tree, x, y, n, diag_add, smem, &flag_sh, red, slots, alpha, &logdet, &quad);
+  if (threadIdx.x != 0) return;
+  if (f != -1) {
+    dev_fail(st, f == SMALL_NONFINITE ? GPRX_NONFINITE_KERNEL : GPRX_CHOLESKY_FAILED, f < 0 ? 0 : f);
+    return;
+  }
+  res[0] = logdet;
+  res[1] = quad;
+  slots_to_grad(slots, GRAD_SLOTS_LEAF + (ARD_D > 0 ? ARD_D : 1) + 1, slot_param, noise, p, res + 2);
+}
+
+template <int ARD_D>
+static cudaError_t launch_small(const HostKernel& k, const double* x, const double* y, int n, double diag_add,
+                                double noise, const int* slot_param, double* alpha, double* res, DevStatus* st,
+                                cudaStream_t s) {
+  const size_t smem = small_smem();
+  cudaError_t e = cudaFuncSetAttribute(small_eval_kernel<ARD_D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  GPRX_LAUNCH(small_eval_kernel<ARD_D>, 1, BT, smem, s, k.tree, x, y, n, diag_add, noise, k.n_params + 1, slot_param,
+              alpha, res, st);
+  return cudaGetLastError();
+}
+
+cudaError_t small_eval(const HostKernel& k, const double* x, const double* y, int n, double diag_add, double noise,
+                       const int* slot_param, double* alpha, double* res, DevStatus* st, cudaStream_t s) {
+  switch (k.ard_d) {
+    case 0: return launch_small<0>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
+    case 4: return launch_small<4>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
+    case 8: return launch_small<8>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
+    case 16: return launch_small<16>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
+    default: return launch_small<32>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
+  }
+}
+
 template <int ARD_D>
 __device__ void cta_eval(const BatchEvalArgs& a, int q, const Work& w, double* smem) {
   __shared__ KTree tree;
@@ -367,6 +532,28 @@ __device__ void cta_eval(const BatchEvalArgs& a, int q, const Work& w, double* s
     return;
   }
   const double noise = noise_sh;
+  if (n <= NB_DIAG) {  // one block: in shared memory throughout
+    int f = 0;
+    double logdet = 0.0, quad = 0.0;
+    for (int attempt = 0; attempt <= a.jit.count; ++attempt) {
+      const double j = attempt == 0 ? 0.0 : a.jit.j[attempt - 1];
+      f = cta_small<ARD_D>(tree, P.x, P.y, n, noise + j, smem, &flag_sh, red, slots, w.alpha, &logdet, &quad);
+      if (f < 0) break;
+    }
+    if (tid == 0) {
+      const double nl = 0.5 * (quad + logdet + (double)n * log(2.0 * M_PI));
+      if (f == SMALL_NONFINITE) a.status[q] = GPRX_NONFINITE_KERNEL;
+      else if (f >= 0) a.status[q] = GPRX_CHOLESKY_FAILED;
+      else {
+        slots_to_grad(slots, GRAD_SLOTS_LEAF + (ARD_D > 0 ? ARD_D : 1) + 1, a.slot_param, noise, p,
+                      a.grad + (long long)q * p);
+        a.nlml[q] = nl;
+        a.status[q] = isfinite(nl) ? GPRX_OK : GPRX_NOT_CONVERGED;
+      }
+    }
+    __syncthreads();
+    return;
+  }
   // fill + factor, retried with the jitter offsets
   int fail = 0;
   for (int attempt = 0; attempt <= a.jit.count; ++attempt) {
@@ -412,14 +599,7 @@ __device__ void cta_eval(const BatchEvalArgs& a, int q, const Work& w, double* s
   if (tid == 0) {
     constexpr int NS = GRAD_SLOTS_LEAF + (ARD_D > 0 ? ARD_D : 1) + 1;
     const double nl = 0.5 * (quad + logdet + (double)n * log(2.0 * M_PI));
-    double* g = a.grad + (long long)q * p;
-    for (int i = 0; i < p; ++i) g[i] = 0.0;
-    for (int s = 0; s < NS - 1; ++s) {
-      const int pi = a.slot_param[s];
-      if (pi >= 0) g[pi] += slots[s];
-    }
-    for (int i = 0; i < p - 1; ++i) g[i] *= -0.5;
-    g[p - 1] = -0.5 * noise * slots[NS - 1];
+    slots_to_grad(slots, NS, a.slot_param, noise, p, a.grad + (long long)q * p);
     a.nlml[q] = nl;
     a.status[q] = isfinite(nl) ? GPRX_OK : GPRX_NOT_CONVERGED;
   }
@@ -443,11 +623,7 @@ __global__ void __launch_bounds__(BT, 1) batch_eval_kernel(BatchEvalArgs a) {
   }
 }
 
-inline size_t batch_smem() {
-  size_t gemm = cg_smem_bytes();
-  size_t tiles = (size_t)(2 * GPRX_MAX_DIM * FT_B + 2 * FT_B + (BT / 32) * 64) * sizeof(double);
-  return std::max(std::max(diag_block_smem(), gemm), tiles);
-}
+inline size_t batch_smem() { return std::max(small_smem(), cg_smem_bytes()); }
 
 // ---------------------------------------------------------------------------
 // per-problem optimizer on the device
@@ -760,9 +936,9 @@ static std::map<std::string, int> g_tune_cache;
 
 gprx_status BatchState::autotune(const double* log_theta_dev, bool force) {
   if (tiles_fixed || (tuned && !force)) return GPRX_OK;
-  cudaDeviceProp prop;
-  GPRX_CUDA_TRY(cudaGetDeviceProperties(&prop, device));
-  const std::string key0 = std::string(prop.name) + "|" + std::to_string(device) + "|" + tree_sig + "|";
+  // the cache lives in this process, so the device's number names it (its
+  // properties took 3 ms to read at the first evaluation of every batch)
+  const std::string key0 = std::to_string(device) + "|" + tree_sig + "|";
   std::vector<std::vector<int>> by_class(BATCH_SIZE_CLASSES);
   for (int q : ord_host) by_class[batch_size_class(n_host[q])].push_back(q);
   if (tune_order.ensure((size_t)std::max(nprob, 1)) != cudaSuccess)

@@ -295,7 +295,7 @@ static __device__ void diag_helpers(double* s, double* tmp, const double* rinv, 
                              long long k0, int nb, double* linv, bool vec, int p, int np, int h, int nh, int sh, int ns,
                              bool tail) {
   const int npad = np * LF, c0 = p * LF, r1 = c0 + LF, q = p - 1;
-  if (sh >= 0) {
+  if (sh >= 0 && linv) {
     const int n_ls = p >= 1 ? 2 : 0, xs_parts = tail ? 4 : 2, n_xs = p >= 2 ? xs_parts : 0;
     for (int t = sh; t < n_ls + n_xs; t += ns) {
       if (t < n_ls) store_l_part(s, ldiag, A, lda, k0, nb, vec, q, t);
@@ -324,47 +324,32 @@ static __device__ void diag_helpers(double* s, double* tmp, const double* rinv, 
   for (int t = h; t < 2 * q; t += nh) inv_x_tile(s, tmp, q, t);
 }
 
-// The whole diagonal-block step for one CTA of FD_THREADS threads: load the
-// nb×nb lower block at (k0, k0) of A, factor it (L back into A), invert it
-// (L⁻¹ into linv, ld NB_DIAG, zero above the diagonal).  fail_sh is a shared
-// int.  Returns the failing column (uniform over the CTA) or −1; either way
-// no copy into shared memory is in flight on return.
-static __device__ int diag_block_factor_inv(double* A, long long lda, long long k0, int nb, double* linv, double* smem,
-                                            int* fail_sh) {
+// Identity padding of the block's lower part up to a multiple of 16.
+static __device__ __forceinline__ void diag_block_pad(double* s, int nb) {
+  const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int npad = (nb + LF - 1) / LF * LF;
+  if (nb < npad)
+    for (int j = warp; j < npad; j += nw)
+      for (int i = j + lane; i < npad; i += 32)
+        if (i >= nb || j >= nb) s[i + j * FLS] = (i == j) ? 1.0 : 0.0;
+}
+
+// Factor and inverse of the nb×nb lower block in s (its column blocks possibly
+// still arriving, one cp.async group each; padded with the identity): L below
+// the diagonal of s, X in the transposed slots, and — unless linv is null — L
+// back to (k0, k0) of A and X to linv (ld NB_DIAG, zero above the diagonal).
+// smem: diag_block_smem() bytes from s on; fail_sh a shared int.  Returns the
+// failing column (uniform over the CTA) or −1.
+static __device__ int diag_block_core(double* A, long long lda, long long k0, int nb, double* linv, bool vec,
+                                      double* smem, int* fail_sh) {
   int& fail = *fail_sh;
   double* s = smem;                  // NB_DIAG × FLS
   double* tmp = s + NB_DIAG * FLS;   // TMP_DOUBLES
   double* rinv = tmp + TMP_DOUBLES;  // NB_DIAG reciprocal pivots
   double* ldiag = rinv + NB_DIAG;    // NB_DIAG diagonal entries of L
-  const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, nw = nt >> 5, lane = tid & 31;
+  const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int npad = (nb + LF - 1) / LF * LF, np = npad / LF;
-  if (tid == 0) fail = -1;
-  // column block q is cp.async group q of every thread (16-byte copies from
-  // the even row at or above the diagonal): blocks 0 and 1 are waited for, the
-  // rest arrives during the first steps
-  const bool vec = ((lda & 1) == 0) && ((((unsigned long long)(A + k0 + k0 * lda)) & 15) == 0);
-  for (int q = 0; q < np; ++q) {
-    for (int j = q * LF + warp; j < q * LF + LF && j < nb; j += nw) {
-      if (vec) {
-        for (int i = (j & ~1) + 2 * lane; i < nb; i += 64) {
-          if (i + 1 < nb) {
-            unsigned sa = (unsigned)__cvta_generic_to_shared(s + i + j * FLS);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(A + (k0 + i) + (k0 + j) * lda));
-          } else {
-            cp_async8(s + i + j * FLS, A + (k0 + i) + (k0 + j) * lda, true);
-          }
-        }
-      } else {
-        for (int i = j + lane; i < nb; i += 32) cp_async8(s + i + j * FLS, A + (k0 + i) + (k0 + j) * lda, true);
-      }
-    }
-    cp_async_commit();
-  }
-  // identity padding (lower part; the copies never reach these entries)
-  if (nb < npad)
-    for (int j = warp; j < npad; j += nw)
-      for (int i = j + lane; i < npad; i += 32)
-        if (i >= nb || j >= nb) s[i + j * FLS] = (i == j) ? 1.0 : 0.0;
+  if (threadIdx.x == 0) fail = -1;
   cp_async_wait_n(np - 2);  // column blocks 0 and 1
   __syncthreads();
   for (int p = 0; p < np; ++p) {
@@ -399,10 +384,44 @@ static __device__ int diag_block_factor_inv(double* A, long long lda, long long 
   // rows of X into linv (all warps)
   diag_helpers(s, tmp, rinv, ldiag, A, lda, k0, nb, linv, vec, np, np, warp, nw, warp, nw, true);
   __syncthreads();
+  if (!linv) return -1;
   // block rows np−1 .. NB_DIAG/16 − 1 (those past the block are zeros)
   for (int t = warp; t < (NB_DIAG / LF - np + 1) * 4; t += nw) store_x_part(s, linv, nb, np - 1 + t / 4, t % 4, 4);
   __syncthreads();
   return -1;
+}
+
+// The whole diagonal-block step for one CTA: load the nb×nb lower block at
+// (k0, k0) of A, factor it (L back into A), invert it (L⁻¹ into linv).  Returns
+// as diag_block_core; either way no copy into shared memory is in flight on
+// return.
+static __device__ int diag_block_factor_inv(double* A, long long lda, long long k0, int nb, double* linv, double* smem,
+                                            int* fail_sh) {
+  double* s = smem;
+  const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, np = (nb + LF - 1) / LF;
+  // column block q is cp.async group q of every thread (16-byte copies from
+  // the even row at or above the diagonal): blocks 0 and 1 are waited for, the
+  // rest arrives during the first steps
+  const bool vec = ((lda & 1) == 0) && ((((unsigned long long)(A + k0 + k0 * lda)) & 15) == 0);
+  for (int q = 0; q < np; ++q) {
+    for (int j = q * LF + warp; j < q * LF + LF && j < nb; j += nw) {
+      if (vec) {
+        for (int i = (j & ~1) + 2 * lane; i < nb; i += 64) {
+          if (i + 1 < nb) {
+            unsigned sa = (unsigned)__cvta_generic_to_shared(s + i + j * FLS);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(A + (k0 + i) + (k0 + j) * lda));
+          } else {
+            cp_async8(s + i + j * FLS, A + (k0 + i) + (k0 + j) * lda, true);
+          }
+        }
+      } else {
+        for (int i = j + lane; i < nb; i += 32) cp_async8(s + i + j * FLS, A + (k0 + i) + (k0 + j) * lda, true);
+      }
+    }
+    cp_async_commit();
+  }
+  diag_block_pad(s, nb);  // the copies never reach these entries
+  return diag_block_core(A, lda, k0, nb, linv, vec, smem, fail_sh);
 }
 
 inline size_t diag_block_smem() { return (size_t)(NB_DIAG * FLS + TMP_DOUBLES + 2 * NB_DIAG) * sizeof(double); }

@@ -204,7 +204,7 @@ gprx_status ExactState::ensure_emu() {
   return GPRX_OK;
 }
 
-gprx_status ExactState::eval(const double* params, double* nlml_out, double* grad) {
+gprx_status ExactState::eval(const double* params, double* nlml_out, double* grad, bool keep_inverse) {
   const int p = num_params();
   std::vector<double> prev(p);
   get_params(prev.data());
@@ -216,7 +216,8 @@ gprx_status ExactState::eval(const double* params, double* nlml_out, double* gra
   js.insert(js.end(), r.begin(), r.end());
   double last = 0.0;
   const size_t nn = (size_t)ld * cap;
-  if (grad && Xinv.n < nn) {
+  const bool small = grad && !keep_inverse && n <= SMALL_EVAL_N && cap == n;
+  if (grad && !small && Xinv.n < nn) {
     size_t half = (size_t)((n + 1) / 2) * ((n + 1) / 2);
     if (Xinv.alloc(nn) != cudaSuccess || scratch.alloc(std::max<size_t>(half, 1)) != cudaSuccess) {
       Xinv.reset();
@@ -230,7 +231,12 @@ gprx_status ExactState::eval(const double* params, double* nlml_out, double* gra
     if ((st = reset_status()) != GPRX_OK) return st;
     const bool emu = grad && use_emu();
     EmuWork ew;
-    if (emu) {
+    if (small) {
+      GPRX_CUDA_TRY(cudaEventRecord(ev[0], stream));
+      GPRX_CUDA_TRY(small_eval(kern, x.p, y.p, n, noise() + j, noise(), slot_param.p, alpha.p, res.p, status.p,
+                               stream));
+      GPRX_CUDA_TRY(cudaEventRecord(ev[4], stream));
+    } else if (emu) {
       // fill, then L and X = L⁻¹ together by recursive halving with the
       // coupling products emulated
       if ((st = ensure_emu()) != GPRX_OK) return st;
@@ -247,7 +253,8 @@ gprx_status ExactState::eval(const double* params, double* nlml_out, double* gra
     } else {
       if ((st = enqueue_factor(j)) != GPRX_OK) return st;
     }
-    if (grad) {
+    if (small) {
+    } else if (grad) {
       // the log-det and α = Xᵀ (X y) run on the side stream beside K⁻¹ = XᵀX:
       // one-CTA and memory-bound kernels next to the products (35 µs off the
       // stream at n = 1537)
@@ -291,6 +298,7 @@ gprx_status ExactState::eval(const double* params, double* nlml_out, double* gra
     DevStatus ds;
     if ((st = read_status(&ds)) != GPRX_OK) return st;
     ev_recorded = true;
+    ev_single = small;
     if (ds.code == GPRX_OK && grad && use_emu() && *emu_err_h.p != 0) {
       write_params(prev.data());
       factor_current();
@@ -334,7 +342,7 @@ gprx_status ExactState::hessian(const double* params, double* out, double* nlml_
   if (online) return set_error(GPRX_INVALID_CONFIG, "an online model takes no hyperparameter evaluation");
   std::vector<double> g(p);
   double v = 0.0;
-  gprx_status st = eval(params, &v, g.data());
+  gprx_status st = eval(params, &v, g.data(), true);
   if (st != GPRX_OK) return st;
   if (nlml_out) *nlml_out = v;
   if (grad_out) std::copy(g.begin(), g.end(), grad_out);
@@ -875,6 +883,12 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
 gprx_status ExactState::stage_times(double* out5) {
   if (!ev_recorded) return set_error(GPRX_INVALID_CONFIG, "no evaluation recorded");
   float ms;
+  if (ev_single) {  // one launch: all of it under the fill's entry
+    GPRX_CUDA_TRY(cudaEventElapsedTime(&ms, ev[0], ev[4]));
+    out5[0] = out5[4] = ms;
+    out5[1] = out5[2] = out5[3] = 0.0;
+    return GPRX_OK;
+  }
   for (int i = 0; i < 4; ++i) {
     GPRX_CUDA_TRY(cudaEventElapsedTime(&ms, ev[i], ev[i + 1]));
     out5[i] = ms;

@@ -76,6 +76,7 @@ struct ExactState {
 
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   bool ev_recorded = false;
+  bool ev_single = false;  // the last evaluation was one launch: ev[0] to ev[4] only
 
   ~ExactState();
   gprx_status create(const double* x, uint64_t n, uint64_t d, const double* y, const gprx_kernel_node* nodes,
@@ -103,7 +104,9 @@ struct ExactState {
   gprx_status factor_with_retries(int stage);
   gprx_status solve_alpha_from_l();
   gprx_status factor_current();
-  gprx_status eval(const double* params, double* nlml, double* grad);
+  // keep_inverse: leave K⁻¹ in A and L⁻¹ in Xinv after a gradient (else a small
+  // problem is evaluated in one launch that keeps neither)
+  gprx_status eval(const double* params, double* nlml, double* grad, bool keep_inverse = false);
   gprx_status nlml(double* out);
   // Hessian of the NLML at params (row-major p × p); the value and the
   // gradient of the same evaluation when nlml_out / grad_out are given

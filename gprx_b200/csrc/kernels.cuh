@@ -53,6 +53,13 @@ cudaError_t cross_contract(const HostKernel& k, const double* z, long long ldz, 
 cudaError_t grad_finalize(const HostKernel& k, const double* partials, int blocks, const int* slot_param_dev,
                           double scale, double noise_coef, double* grad, DevStatus* st, cudaStream_t s);
 
+// One evaluation of at most SMALL_EVAL_N points in one launch (batch.cu): x is
+// n×d with leading dimension n; res[0] = log-det, res[1] = yᵀα, res[2 ..] the
+// gradient; α to alpha.  A failed factor or a non-finite kernel value goes to st.
+constexpr int SMALL_EVAL_N = 128;
+cudaError_t small_eval(const HostKernel& k, const double* x, const double* y, int n, double diag_add, double noise,
+                       const int* slot_param, double* alpha, double* res, DevStatus* st, cudaStream_t s);
+
 // Maximum partial-block count of grad_contract (sizes the partials buffer).
 int grad_max_blocks();
 
