@@ -301,22 +301,24 @@ __device__ inline bool in_default_interval(double log_v) {
 }
 
 // LLT of the lower n×n matrix in w.A with the diagonal-block inverses in
-// w.linv.  Returns the failing column or −1.
+// w.linv, left-looking: block column k takes all earlier panels in one product
+// (K = k0), so its entries are read and written once instead of once per
+// earlier column (one CTA has no trailing parallelism to gain from the
+// right-looking order).  Returns the failing column or −1.
 __device__ int cta_potrf(const Work& w, int n, long long ld, double* smem, int* fail_sh, int cfg) {
   for (int k0 = 0; k0 < n; k0 += NB_DIAG) {
     const int nbk = min(NB_DIAG, n - k0);
+    double* Akk = w.A + k0 + (long long)k0 * ld;
+    if (k0 > 0)
+      cta_gemm<false, true>(cfg, n - k0, nbk, k0, w.A + k0, ld, w.A + k0, ld, Akk, ld, -1.0, 1.0, true, CG_FULL, smem);
     double* lk = w.linv + (long long)(k0 / NB_DIAG) * NB_DIAG * NB_DIAG;
     const int f = diag_block_factor_inv(w.A, ld, k0, nbk, lk, smem, fail_sh);
     if (f >= 0) return k0 + f;
     const int rest = n - k0 - nbk;
     if (rest <= 0) break;
-    double* P = w.A + (k0 + nbk) + (long long)k0 * ld;
     // P := P L_kk⁻ᵀ (in place: one tile must span all nbk columns)
-    cta_gemm<false, true>(nbk <= cg_tile_n(cfg) ? cfg : 0, rest, nbk, nbk, P, ld, lk, NB_DIAG, P, ld, 1.0, 0.0, false,
-                          CG_FULL, smem);
-    // A22 −= P Pᵀ (lower)
-    double* A22 = w.A + (k0 + nbk) + (long long)(k0 + nbk) * ld;
-    cta_gemm<false, true>(cfg, rest, rest, nbk, P, ld, P, ld, A22, ld, -1.0, 1.0, true, CG_FULL, smem);
+    cta_gemm<false, true>(nbk <= cg_tile_n(cfg) ? cfg : 0, rest, nbk, nbk, Akk + nbk, ld, lk, NB_DIAG, Akk + nbk, ld,
+                          1.0, 0.0, false, CG_TO_COL, smem);
   }
   return -1;
 }
@@ -335,7 +337,7 @@ __device__ void cta_trtri(const Work& w, int n, long long ld, double* smem, int 
     // T = L_i,<i X_<i,<i  (X lower: k from the tile's first column)
     cta_gemm<false, false>(cfg, nbi, r0, r0, w.A + r0, ld, w.X, ld, w.T, NB_DIAG, 1.0, 0.0, false, CG_FROM_COL, smem);
     // X_i,<i = −L_ii⁻¹ T
-    cta_gemm<false, false>(cfg, nbi, r0, nbi, li, NB_DIAG, w.T, NB_DIAG, w.X + r0, ld, -1.0, 0.0, false, CG_FULL,
+    cta_gemm<false, false>(cfg, nbi, r0, nbi, li, NB_DIAG, w.T, NB_DIAG, w.X + r0, ld, -1.0, 0.0, false, CG_TO_ROW,
                            smem);
   }
   __syncthreads();

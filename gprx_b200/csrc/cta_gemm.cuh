@@ -24,8 +24,11 @@
 // skipped and warps whose block is wholly above it only help load.
 // kmode: CG_FULL kb = 0; CG_FROM_ROW kb = the tile's first row (opA(i,k) = 0
 // for k < i); CG_FROM_COL kb = the tile's first column (opB(k,j) = 0 for
-// k < j).  A tile reads all its inputs before it writes C, so C may alias A's
-// rows when one tile spans all of N.
+// k < j); CG_TO_ROW the k range ends at the tile's last row (opA(i,k) = 0 for
+// k > i); CG_TO_COL each warp's ends at its own last column (opB(k,j) = 0 for
+// k > j; a scheduler's warps hold different columns, so it saves DMMA time where
+// one tile spans the triangle).  A tile reads all its inputs before it writes C,
+// so C may alias A's rows when one tile spans all of N.
 #pragma once
 
 #include "gemm_f64.cuh"
@@ -33,7 +36,7 @@
 namespace gprx {
 
 constexpr int CG_THREADS = 512;
-constexpr int CG_FULL = 0, CG_FROM_ROW = 1, CG_FROM_COL = 2;
+constexpr int CG_FULL = 0, CG_FROM_ROW = 1, CG_FROM_COL = 2, CG_TO_ROW = 3, CG_TO_COL = 4;
 
 // tile shapes (TM × TN, k chunk TK, warp grid WGM × WGN, copy-ring stages ST)
 // by configuration index; the 64×128 tile takes 64-deep chunks in two stages
@@ -113,7 +116,8 @@ __device__ void cta_gemm_tile(int M, int N, int K, const double* A, long long ld
     return kb < K ? kb : K;
   };
   auto tile_nch = [&](int t) {
-    const int n = (K - tile_kb(t) + CG_K - 1) / CG_K;
+    const int ke = kmode == CG_TO_ROW ? min(K, (t % tm_n) * CG_M + CG_M) : K;
+    const int n = (ke - tile_kb(t) + CG_K - 1) / CG_K;
     return n > 0 ? n : 1;  // an empty k range still runs one zero chunk
   };
   auto next_used = [&](int t) {
@@ -225,6 +229,7 @@ __device__ void cta_gemm_tile(int M, int N, int K, const double* A, long long ld
       for (int nj = 0; nj < NJ; ++nj)
 #pragma unroll
         for (int r = 0; r < 4; ++r) acc[mi][nj][r] = 0.0;
+    const int klim = kmode == CG_TO_COL ? n0 + wn * WN + WN : K;  // (CG_TO_COL: kb = 0)
     for (int c = 0; c < nch; ++c, ++gch) {
       cp_async_wait<ST - 2>();
       __syncthreads();
@@ -234,6 +239,7 @@ __device__ void cta_gemm_tile(int M, int N, int K, const double* A, long long ld
         const double* sB = sA + SA::ELEMS;
 #pragma unroll
         for (int kk = 0; kk < CG_K; kk += 4) {
+          if (kmode == CG_TO_COL && c * CG_K + kk >= klim) break;
           double a[MI][2], b[NJ];
 #pragma unroll
           for (int mi = 0; mi < MI; ++mi) {
