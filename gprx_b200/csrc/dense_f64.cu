@@ -778,47 +778,58 @@ cudaError_t trmv_lower(const double* X, long long ld, int n, const double* y, do
   return cudaGetLastError();
 }
 
-__global__ void gemv_t_kernel(const double* M, long long ld, int nrows, int ncols, bool lower, const double* v,
-                              double* out, const DevStatus* st) {
+// Sum over one column: a warp's lanes or (BLOCK) a whole CTA of 256 threads;
+// the first thread of the group gets it.
+template <bool BLOCK>
+__device__ __forceinline__ double column_sum(double acc) {
+  __shared__ double red[32];
+  return BLOCK ? block_sum(acc, red) : warp_sum(acc);
+}
+
+template <bool BLOCK>
+__global__ void __launch_bounds__(256) gemv_t_kernel(const double* M, long long ld, int nrows, int ncols, bool lower,
+                                                     const double* v, double* out, const DevStatus* st) {
+  constexpr int G = BLOCK ? 256 : 32;
   if (dev_failed(st)) return;
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (warp >= ncols) return;
-  const double* col = M + (long long)warp * ld;
-  int i0 = lower ? warp : 0;
+  const int c = (blockIdx.x * 256 + threadIdx.x) / G, t = threadIdx.x % G;
+  if (c >= ncols) return;
+  const double* col = M + (long long)c * ld;
   double acc = 0.0;
-  for (int i = i0 + lane; i < nrows; i += 32) acc = fma(col[i], v[i], acc);
-  acc = warp_sum(acc);
-  if (lane == 0) out[warp] = acc;
+  for (int i = (lower ? c : 0) + t; i < nrows; i += G) acc = fma(col[i], v[i], acc);
+  acc = column_sum<BLOCK>(acc);
+  if (t == 0) out[c] = acc;
 }
 
 cudaError_t gemv_t(const double* M, long long ld, int nrows, int ncols, bool lower, const double* v, double* out,
-                   DevStatus* st, cudaStream_t s) {
+                   DevStatus* st, cudaStream_t s, bool block) {
   if (ncols <= 0) return cudaSuccess;
-  GPRX_LAUNCH(gemv_t_kernel, ceil_div((long long)ncols * 32, 256), 256, 0, s, M, ld, nrows, ncols, lower, v, out, st);
+  if (block) GPRX_LAUNCH(gemv_t_kernel<true>, ncols, 256, 0, s, M, ld, nrows, ncols, lower, v, out, st);
+  else GPRX_LAUNCH(gemv_t_kernel<false>, ceil_div((long long)ncols * 32, 256), 256, 0, s, M, ld, nrows, ncols, lower, v, out, st);
   return cudaGetLastError();
 }
 
-__global__ void col_sumsq_kernel(const double* M, long long ld, int nrows, int ncols, const double* w, double* out,
-                                 const DevStatus* st) {
+template <bool BLOCK>
+__global__ void __launch_bounds__(256) col_sumsq_kernel(const double* M, long long ld, int nrows, int ncols,
+                                                        const double* w, double* out, const DevStatus* st) {
+  constexpr int G = BLOCK ? 256 : 32;
   if (dev_failed(st)) return;
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (warp >= ncols) return;
-  const double* col = M + (long long)warp * ld;
+  const int c = (blockIdx.x * 256 + threadIdx.x) / G, t = threadIdx.x % G;
+  if (c >= ncols) return;
+  const double* col = M + (long long)c * ld;
   double acc = 0.0;
-  for (int i = lane; i < nrows; i += 32) {
-    double v = col[i];
+  for (int i = t; i < nrows; i += G) {
+    const double v = col[i];
     acc = w ? fma(v, v / w[i], acc) : fma(v, v, acc);
   }
-  acc = warp_sum(acc);
-  if (lane == 0) out[warp] = acc;
+  acc = column_sum<BLOCK>(acc);
+  if (t == 0) out[c] = acc;
 }
 
 cudaError_t col_sumsq(const double* M, long long ld, int nrows, int ncols, const double* w, double* out,
-                      DevStatus* st, cudaStream_t s) {
+                      DevStatus* st, cudaStream_t s, bool block) {
   if (ncols <= 0) return cudaSuccess;
-  GPRX_LAUNCH(col_sumsq_kernel, ceil_div((long long)ncols * 32, 256), 256, 0, s, M, ld, nrows, ncols, w, out, st);
+  if (block) GPRX_LAUNCH(col_sumsq_kernel<true>, ncols, 256, 0, s, M, ld, nrows, ncols, w, out, st);
+  else GPRX_LAUNCH(col_sumsq_kernel<false>, ceil_div((long long)ncols * 32, 256), 256, 0, s, M, ld, nrows, ncols, w, out, st);
   return cudaGetLastError();
 }
 

@@ -95,12 +95,14 @@ cudaError_t logdet_diag(const double* L, long long ld, int n, bool ldlt, double*
 // z = X y for lower-triangular X (n×n, ld).
 cudaError_t trmv_lower(const double* X, long long ld, int n, const double* y, double* z, DevStatus* st,
                        cudaStream_t s);
-// out_j = Σ_{i ≥ (lower ? j : 0)} M(i,j) v_i  for j < ncols (one warp per column).
+// out_j = Σ_{i ≥ (lower ? j : 0)} M(i,j) v_i  for j < ncols: one warp per
+// column, or (block) one CTA, for few long columns: 12 → 4 µs for one of 1000,
+// 36 → 8 µs for the squares over D of four of 2000.  The sums differ in bits.
 cudaError_t gemv_t(const double* M, long long ld, int nrows, int ncols, bool lower, const double* v, double* out,
-                   DevStatus* st, cudaStream_t s);
+                   DevStatus* st, cudaStream_t s, bool block = false);
 // out_j = Σ_i M(i,j)² (/ w_i when w != nullptr) for j < ncols.
 cudaError_t col_sumsq(const double* M, long long ld, int nrows, int ncols, const double* w, double* out,
-                      DevStatus* st, cudaStream_t s);
+                      DevStatus* st, cudaStream_t s, bool block = false);
 
 // out = Σ_i a_i b_i (single block, deterministic).
 cudaError_t dot_dev(const double* a, const double* b, int n, double* out, DevStatus* st, cudaStream_t s);

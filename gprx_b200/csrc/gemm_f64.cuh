@@ -30,6 +30,10 @@ enum GemmMode : int {
   GEMM_K_TO_COL = 32,   // k-loop stops at the tile's last global column + 1 (op(B)(k, j) = 0 for k > j)
 };
 
+// K_TO_ROW products of at most this many tiles walk row by row from the last
+// (longest) row; larger ones keep the column order, whose tiles share B in L2.
+constexpr int GEMM_ROWS_FIRST_TILES = 4096;
+
 struct GemmParams {
   int M, N, K;
   const double* A;
@@ -48,7 +52,7 @@ struct GemmParams {
   // batched: pointer strides per blockIdx.z when splits == 1 and batch > 1
   long long strideA, strideB, strideC;
   int max_ctas;             // > 0: at most this many CTAs, each looping over tiles
-  int splits_tiles;         // set by the launcher: tile count when max_ctas > 0
+  int splits_tiles;         // set by the launcher: tile count
 };
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {
@@ -107,7 +111,8 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES, TA, TB>::T
   if (p.mode & GEMM_LOWER_TILES) {
     // tile_idx enumerates (tm, tn) with the tile not strictly above the
     // diagonal; when row0 == col0 and BM == BN that is tn ≤ tm.
-    int idx = tile_idx;
+    // tiles with the longest k range first: the last wave is then of short ones
+    int idx = (p.mode & GEMM_K_TO_COL) ? p.splits_tiles - 1 - tile_idx : tile_idx;
     // general enumeration: walk columns; tile (tm, tn) is kept when its last
     // global row ≥ its first global column.
     const int tiles_n = (p.N + BN - 1) / BN;
@@ -124,6 +129,10 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES, TA, TB>::T
       idx -= cnt;
     }
     if (tile_m < 0) return;
+  } else if ((p.mode & GEMM_K_TO_ROW) && p.splits_tiles <= GEMM_ROWS_FIRST_TILES) {
+    const int tiles_n = (p.N + BN - 1) / BN;  // longest k range (last rows) first
+    tile_m = tiles_m - 1 - tile_idx / tiles_n;
+    tile_n = tile_idx % tiles_n;
   } else {
     tile_m = tile_idx % tiles_m;
     tile_n = tile_idx / tiles_m;

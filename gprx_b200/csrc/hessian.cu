@@ -398,12 +398,16 @@ __global__ void __launch_bounds__(HESS_THREADS) fill_deriv_kernel(KTree t, HessM
   }
 }
 
-// out[q] = Σ_b partials[b·stride + q] for q < nq (fixed order).
+// out[q] = Σ_b partials[b·stride + q] for q < nq (fixed order): a warp per
+// slot, lanes over the blocks (a thread per slot took 82 µs at n = 2048).
+constexpr int REDUCE_THREADS = 1024;
 __global__ void reduce_slots_kernel(const double* partials, int blocks, int stride, int nq, double* out) {
-  for (int q = threadIdx.x; q < nq; q += blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < nq; q += REDUCE_THREADS / 32) {
     double s = 0.0;
-    for (int b = 0; b < blocks; ++b) s += partials[(long long)b * stride + q];
-    out[q] = s;
+    for (int b = lane; b < blocks; b += 32) s += partials[(long long)b * stride + q];
+    s = warp_sum(s);
+    if (lane == 0) out[q] = s;
   }
 }
 
@@ -486,7 +490,7 @@ cudaError_t fill_deriv(const HostKernel& k, const HessMap& hm, int i, const doub
 }
 
 cudaError_t reduce_slots(const double* partials, int blocks, int stride, int nq, double* out, cudaStream_t s) {
-  GPRX_LAUNCH(reduce_slots_kernel, 1, 64, 0, s, partials, blocks, stride, nq, out);
+  GPRX_LAUNCH(reduce_slots_kernel, 1, REDUCE_THREADS, 0, s, partials, blocks, stride, nq, out);
   return cudaGetLastError();
 }
 
