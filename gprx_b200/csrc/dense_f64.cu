@@ -205,16 +205,24 @@ cudaError_t FactorCtx::ensure(int nblk) {
 // the chain's panel products: K ≤ NB, N ≤ NB
 // ---------------------------------------------------------------------------
 // C(M×N) = alpha · A(M×K) · B(N×K)ᵀ + beta · C with A(i,k) = A[i + k·lda],
-// B(j,k) = B[j + k·ldb], C column-major; lower: only i ≥ j is written.  One
-// CTA of 256 threads per PG_TM-row strip stages the strip of A and all of B
-// in shared memory in one go (K is one panel: no k pipeline, one memory
+// B(j,k) = B[j + k·ldb], C column-major; lower: only i ≥ j is written; tri: B is
+// lower triangular (B(j,k) = 0 for k > j), so a warp's k range ends at its last
+// column.  One CTA of 256 threads per TM-row strip stages the strip of A and all
+// of B in shared memory in one go (K is one panel: no k pipeline, one memory
 // latency instead of one per k chunk), prefetches its C values meanwhile,
 // then runs the DMMA k steps.  A strip is read whole before it is written,
 // so C may be A's rows when beta = 0 (the in-place panel solve).
+//
+// TM = 16 while the strips fit one wave of SMs (M ≤ 16·148), else 32: a strip of
+// 32 rows holds its SM's DMMA pipe for 8192 cycles (4.2 µs), one of 16 rows for
+// 4096, for 2304 with a triangular B.  Each scheduler gets two warps whose column
+// blocks add up to the same k steps.
 constexpr int PG_TM = 32;
-constexpr int PG_LDA = PG_TM + 4;  // ≡ 4 mod 16 doubles: conflict-free fragments
 constexpr int PG_LDB = NB + 4;
-inline size_t panel_gemm_smem() { return (size_t)(NB * PG_LDA + NB * PG_LDB) * sizeof(double); }
+template <int TM>
+constexpr int pg_lda() { return TM + 4; }  // ≡ 4 mod 16 doubles: conflict-free fragments
+template <int TM>
+inline size_t panel_gemm_smem() { return (size_t)(NB * pg_lda<TM>() + NB * PG_LDB) * sizeof(double); }
 
 struct PanelGemmArgs {
   int M, N, K;
@@ -225,35 +233,37 @@ struct PanelGemmArgs {
   double* C;
   long long ldc;
   double alpha, beta;
-  int lower;
+  int lower, tri;
   const DevStatus* st;
 };
 
+template <int TM>
 __global__ void __launch_bounds__(256) panel_gemm_kernel(PanelGemmArgs g) {
+  constexpr int LDA = pg_lda<TM>(), NJ = TM / 8;  // warps: 16 rows × 8·NJ columns
   extern __shared__ __align__(16) double smem[];
   chain_dependency_wait_and_release();
   if (dev_failed(g.st)) return;
-  double* sA = smem;                 // [k][i], ld PG_LDA
-  double* sB = smem + NB * PG_LDA;   // [k][j], ld PG_LDB
+  double* sA = smem;             // [k][i], ld LDA
+  double* sB = smem + NB * LDA;  // [k][j], ld PG_LDB
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t4 = lane & 3;
-  const int m0 = blockIdx.x * PG_TM;
+  const int m0 = blockIdx.x * TM;
   const int KP = (g.K + 3) & ~3;
   const bool a16 = ((g.lda & 1) == 0) && ((reinterpret_cast<unsigned long long>(g.A) & 15) == 0);
   const bool b16 = ((g.ldb & 1) == 0) && ((reinterpret_cast<unsigned long long>(g.B) & 15) == 0);
-  // A strip: PG_TM × KP (zero past M and K)
+  // A strip: TM × KP (zero past M and K)
   if (a16) {
-    for (int e = tid; e < (PG_TM / 2) * KP; e += 256) {
-      const int i = 2 * (e % (PG_TM / 2)), k = e / (PG_TM / 2), gi = m0 + i;
+    for (int e = tid; e < (TM / 2) * KP; e += 256) {
+      const int i = 2 * (e % (TM / 2)), k = e / (TM / 2), gi = m0 + i;
       const int bytes = (gi < g.M && k < g.K) ? (gi + 1 < g.M ? 16 : 8) : 0;
-      const unsigned d = (unsigned)__cvta_generic_to_shared(sA + k * PG_LDA + i);
+      const unsigned d = (unsigned)__cvta_generic_to_shared(sA + k * LDA + i);
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d),
                    "l"(bytes ? g.A + gi + (long long)k * g.lda : g.A), "r"(bytes));
     }
   } else {
-    for (int e = tid; e < PG_TM * KP; e += 256) {
-      const int i = e % PG_TM, k = e / PG_TM, gi = m0 + i;
+    for (int e = tid; e < TM * KP; e += 256) {
+      const int i = e % TM, k = e / TM, gi = m0 + i;
       const bool ok = gi < g.M && k < g.K;
-      cp_async8(sA + k * PG_LDA + i, ok ? g.A + gi + (long long)k * g.lda : g.A, ok);
+      cp_async8(sA + k * LDA + i, ok ? g.A + gi + (long long)k * g.lda : g.A, ok);
     }
   }
   // B: NB × KP (zero past N and K)
@@ -273,13 +283,15 @@ __global__ void __launch_bounds__(256) panel_gemm_kernel(PanelGemmArgs g) {
     }
   }
   cp_async_commit();
-  // warps in a 2 × 4 grid of 16 × 32 blocks (MI = 1, NJ = 4)
-  const int wm = warp & 1, wn = warp >> 1;
-  const int rb = wm * 16, cb = wn * 32;
+  // TM = 32: a 2 × 4 grid of 16 × 32 blocks, columns 0 1 3 2; TM = 16: eight
+  // blocks of 16 × 16, columns 0 1 2 3 7 6 5 4 (warps w and w + 4 share a scheduler)
+  const int wm = TM == 32 ? warp & 1 : 0, w = TM == 32 ? warp >> 1 : warp;
+  const int wn = TM == 32 ? (w < 2 ? w : 5 - w) : (w < 4 ? w : 11 - w);
+  const int rb = wm * 16, cb = wn * 8 * NJ;
   const bool wskip = (cb >= g.N) || (g.lower && m0 + rb + 15 < cb);
-  double cv[4][4];
+  double cv[NJ][4];
 #pragma unroll
-  for (int nj = 0; nj < 4; ++nj)
+  for (int nj = 0; nj < NJ; ++nj)
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int row = m0 + rb + gq + ((r & 2) ? 8 : 0), col = cb + nj * 8 + 2 * t4 + (r & 1);
@@ -289,23 +301,24 @@ __global__ void __launch_bounds__(256) panel_gemm_kernel(PanelGemmArgs g) {
   cp_async_wait<0>();
   __syncthreads();
   if (wskip) return;
-  double acc[4][4];
+  double acc[NJ][4];
 #pragma unroll
-  for (int nj = 0; nj < 4; ++nj)
+  for (int nj = 0; nj < NJ; ++nj)
 #pragma unroll
     for (int r = 0; r < 4; ++r) acc[nj][r] = 0.0;
+  const int ke = g.tri ? min(KP, cb + 8 * NJ) : KP;
 #pragma unroll 4
-  for (int kk = 0; kk < KP; kk += 4) {
-    const double a0 = sA[(kk + t4) * PG_LDA + rb + gq];
-    const double a1 = sA[(kk + t4) * PG_LDA + rb + gq + 8];
-    double b[4];
+  for (int kk = 0; kk < ke; kk += 4) {
+    const double a0 = sA[(kk + t4) * LDA + rb + gq];
+    const double a1 = sA[(kk + t4) * LDA + rb + gq + 8];
+    double b[NJ];
 #pragma unroll
-    for (int nj = 0; nj < 4; ++nj) b[nj] = sB[(kk + t4) * PG_LDB + cb + nj * 8 + gq];
+    for (int nj = 0; nj < NJ; ++nj) b[nj] = sB[(kk + t4) * PG_LDB + cb + nj * 8 + gq];
 #pragma unroll
-    for (int nj = 0; nj < 4; ++nj) dmma_16x8x4(acc[nj], a0, a1, b[nj]);
+    for (int nj = 0; nj < NJ; ++nj) dmma_16x8x4(acc[nj], a0, a1, b[nj]);
   }
 #pragma unroll
-  for (int nj = 0; nj < 4; ++nj)
+  for (int nj = 0; nj < NJ; ++nj)
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int row = m0 + rb + gq + ((r & 2) ? 8 : 0), col = cb + nj * 8 + 2 * t4 + (r & 1);
@@ -336,20 +349,27 @@ static cudaError_t launch_chain(void (*kernel)(Params...), dim3 grid, dim3 block
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-static cudaError_t panel_gemm(int M, int N, int K, const double* A, long long lda, const double* B, long long ldb,
-                              double* C, long long ldc, double alpha, double beta, bool lower, const DevStatus* st,
-                              cudaStream_t s, bool chained = false) {
+template <int TM>
+static cudaError_t panel_gemm_launch(const PanelGemmArgs& g, cudaStream_t s, bool chained) {
   static bool attr = false;
   if (!attr) {
-    CK(cudaFuncSetAttribute(panel_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_gemm_smem()));
+    CK(cudaFuncSetAttribute(panel_gemm_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)panel_gemm_smem<TM>()));
     attr = true;
   }
+  if (chained)
+    return launch_chain(panel_gemm_kernel<TM>, dim3(ceil_div(g.M, TM)), dim3(256), panel_gemm_smem<TM>(), s, g);
+  GPRX_LAUNCH(panel_gemm_kernel<TM>, ceil_div(g.M, TM), 256, panel_gemm_smem<TM>(), s, g);
+  return cudaGetLastError();
+}
+
+static cudaError_t panel_gemm(int M, int N, int K, const double* A, long long lda, const double* B, long long ldb,
+                              double* C, long long ldc, double alpha, double beta, bool lower, bool tri,
+                              const DevStatus* st, cudaStream_t s, bool chained = false) {
   if (M <= 0 || N <= 0) return cudaSuccess;
   if (N > NB || K > NB || K < 0) return cudaErrorInvalidValue;
-  PanelGemmArgs g{M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, lower ? 1 : 0, st};
-  if (chained) return launch_chain(panel_gemm_kernel, dim3(ceil_div(M, PG_TM)), dim3(256), panel_gemm_smem(), s, g);
-  GPRX_LAUNCH(panel_gemm_kernel, ceil_div(M, PG_TM), 256, panel_gemm_smem(), s, g);
-  return cudaGetLastError();
+  const PanelGemmArgs g{M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, lower ? 1 : 0, tri ? 1 : 0, st};
+  return M <= 16 * 148 ? panel_gemm_launch<16>(g, s, chained) : panel_gemm_launch<PG_TM>(g, s, chained);
 }
 
 // rows below the diagonal block up to which the chain uses dependent launch
@@ -377,7 +397,7 @@ static cudaError_t diag_and_panel(double* A, long long ld, int n, int k0, double
     // a strip is staged whole before it is written); after an event wait the
     // launch is a plain one
     if (before_panel) CK(cudaStreamWaitEvent(s, before_panel, 0));
-    CK(panel_gemm(rest, nbk, nbk, P, ld, lk, NB, P, ld, 1.0, 0.0, false, st, s, chained && !before_panel));
+    CK(panel_gemm(rest, nbk, nbk, P, ld, lk, NB, P, ld, 1.0, 0.0, false, true, st, s, chained && !before_panel));
   }
   return cudaGetLastError();
 }
@@ -433,12 +453,13 @@ cudaError_t potrf_blocked(double* A, long long ld, int n, double* linv, DevStatu
     if (m > NB) {
       if (k >= 1) CK(cudaStreamWaitEvent(X2, Es[k - 1], 0));
       CK(cudaStreamWaitEvent(X2, Ep[k], 0));
-      CK(panel_gemm(m - NB, w, NB, Pk + NB, ld, Pk, ld, A + (c1 + NB) + (long long)c1 * ld, ld, -1.0, 1.0, false, st,
-                    X2));
+      CK(panel_gemm(m - NB, w, NB, Pk + NB, ld, Pk, ld, A + (c1 + NB) + (long long)c1 * ld, ld, -1.0, 1.0, false,
+                    false, st, X2));
       CK(cudaEventRecord(Ec[k], X2));
       lower_done = Ec[k];
     }
-    CK(panel_gemm(min(m, NB), w, NB, Pk, ld, Pk, ld, A + c1 + (long long)c1 * ld, ld, -1.0, 1.0, true, st, X));
+    CK(panel_gemm(min(m, NB), w, NB, Pk, ld, Pk, ld, A + c1 + (long long)c1 * ld, ld, -1.0, 1.0, true, false, st,
+                  X));
     CK(diag_and_panel(A, ld, n, c1, linv, st, X, lower_done));
     CK(cudaEventRecord(Ep[k + 1], X));
     last = k + 1;
