@@ -10,7 +10,8 @@
 // 128×128 products on DMMA and one store.  The cluster barrier orders the
 // steps: CTAs of one cluster are co-resident, so nothing spins.
 //
-// What bounds it: for one strip the chain (about 2 µs a block); for many
+// What bounds it: for one strip the chain and the tile that each CTA folds a step
+// (5 µs a block measured; a 128×128 tile alone is 2048 cycles of DMMA); for many
 // strips the reads of L, n²/2 values per strip out of L2.  The two-product
 // form it replaces took two launches of one to n/128 tiles of 128×128 for
 // every block: 33 µs each with one right-hand side, 16 blocks = 1.05 ms at
@@ -52,6 +53,12 @@ inline size_t ts_smem(int NT, int own, bool one) {
                            (size_t)own * (one ? NB : NT * 4 * TS_THREADS));
 }
 
+// v to CTA `rank` of the cluster at shared address `addr` (of this CTA's layout)
+__device__ __forceinline__ void cluster_store(unsigned addr, int rank, double v) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
@@ -245,12 +252,15 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(TriSolveArgs g
 // The same steps on FP64 FMAs: a DMMA spends seven eighths of its columns on
 // one right-hand side (2 K cycles a 128×128 tile, 16 FMA a cycle and scheduler
 // either way), here a tile costs 64 FMAs a thread.  L_{s+1,s} waits in
-// registers, the diagonal block's inverse in shared memory.  Forward, a thread
+// registers, the diagonal block's inverse in shared memory, and the owner writes
+// x_s into every CTA's shared memory (a read back from L2 and the store's way
+// there were a third of the step).  Forward, a thread
 // owns a row and half of the k range (column-major L: coalesced over rows);
 // transposed, a warp owns 16 rows of Lᵀ, its lanes run along k, and a
 // reduce-scatter of 16 shuffles leaves row ii in lanes 2·ii, 2·ii + 1.
-// Measured (forward / transposed, µs, DMMA → FMA): n = 512 23 / 23 → 18 / 18,
-// n = 2000 83 / 83 → 59 / 55, n = 4096 229 / 201 → 151 / 127.
+// Bound by the reads of L at 16 SMs' rate and the chain.  Measured (forward /
+// transposed, µs, on DMMA → here): n = 512 23 / 23 → 17 / 17, n = 2000 82 / 82 →
+// 53 / 46, n = 4096 227 / 201 → 151 / 110.
 struct TriVecArgs {
   const double* L;
   long long ld;
@@ -263,7 +273,7 @@ struct TriVecArgs {
   const DevStatus* st;
 };
 
-inline size_t tv_smem(int own) { return sizeof(double) * ((size_t)NB * NB + 4 * NB + (size_t)own * NB); }
+inline size_t tv_smem(int own) { return sizeof(double) * ((size_t)NB * NB + 6 * NB + (size_t)own * NB); }
 
 // v[ii] of 32 lanes summed; lane l returns row l / 2.
 __device__ __forceinline__ double scatter16(double (&v)[16]) {
@@ -285,8 +295,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_vec_kernel(TriVecArgs g) {
   extern __shared__ __align__(16) double ts_sm[];
   if (dev_failed(g.st)) return;  // the same word for the whole cluster
   double* li = ts_sm;           // the owned diagonal block's inverse, ld NB
-  double* xs = li + NB * NB;    // x_s
-  double* bs = xs + NB;         // right-hand side of the owned block
+  double* xbuf = li + NB * NB;  // x_s in slot s mod 3, written by the owner into every CTA
+  double* bs = xbuf + 3 * NB;   // right-hand side of the owned block
   double* part = bs + NB;       // [half][row]
   double* sums = part + 2 * NB;  // [owned block][row]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -296,6 +306,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_vec_kernel(TriVecArgs g) {
   const int own = (nblk - rank + C - 1) / C;
   for (int e = tid; e < own * NB; e += TS_THREADS) sums[e] = 0.0;
   double f[64];
+  double bown = 0.0;  // row tid of the owned block's right-hand side
   auto load_tile = [&](int i0, int k0) {
 #pragma unroll
     for (int u = 0; u < 64; ++u) {
@@ -307,17 +318,21 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_vec_kernel(TriVecArgs g) {
       }
     }
   };
-  auto prefetch = [&](int s) {
+  // the inverse and the right-hand side of the CTA's next block, as soon as the
+  // one before is solved (they depend on nobody)
+  auto stage_block = [&](int s) {
+    if (s >= nblk) return;
     const double* src = g.linv + (long long)(first(s) / NB) * NB * NB;
     for (int e = 2 * tid; e < NB * NB; e += 2 * TS_THREADS) {
       const unsigned d = (unsigned)__cvta_generic_to_shared(li + e);
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + e));
     }
     cp_async_commit();
-    if (s > 0) load_tile(first(s), first(s - 1));
+    bown = tid < NB && first(s) + tid < n ? g.b[first(s) + tid] : 0.0;
   };
   // (tile in f) · x into the sums of owned block o
   auto fold = [&](int o, int i0, int s) {
+    const double* xs = xbuf + (s % 3) * NB;
     if (TRANS) {
       double v[16], x[4];
 #pragma unroll
@@ -349,7 +364,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_vec_kernel(TriVecArgs g) {
     const int i0 = first(s), o = s / C;
     cp_async_wait<0>();
     __syncthreads();
-    if (tid < NB) bs[tid] = i0 + tid < n ? g.b[i0 + tid] - sums[o * NB + tid] : 0.0;
+    if (tid < NB) bs[tid] = bown - sums[o * NB + tid];  // zero past n: both terms are
     __syncthreads();
     if (TRANS) {  // Σ_{k ≥ i} X(k, i) b_k
       double v[16], x[4];
@@ -363,8 +378,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_vec_kernel(TriVecArgs g) {
           if (32 * u + 31 >= 16 * warp) v[i] = fma(li[(16 * warp + i) * NB + lane + 32 * u], x[u], v[i]);
       }
       const double t = scatter16(v);
-      const int i = i0 + 16 * warp + (lane >> 1);
-      if (!(lane & 1) && i < n) g.b[i] = t;
+      if (!(lane & 1)) part[16 * warp + (lane >> 1)] = t;
+      __syncthreads();
     } else {  // Σ_{k ≤ i} X(i, k) b_k
       double a[4] = {0, 0, 0, 0};
       const int end = min(64, (row | 31) + 1 - kb);
@@ -379,38 +394,51 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_vec_kernel(TriVecArgs g) {
       }
       part[tid] = (a[0] + a[1]) + (a[2] + a[3]);
       __syncthreads();
-      if (tid < NB && i0 + tid < n) g.b[i0 + tid] = part[tid] + part[NB + tid];
+      if (tid < NB) part[tid] += part[NB + tid];
+    }
+    // x_s into every CTA's buffer
+    if (tid < NB) {
+      const unsigned at = (unsigned)__cvta_generic_to_shared(xbuf + (s % 3) * NB + tid);
+      if (s + 1 < nblk)
+        for (int c = 0; c < C; ++c) cluster_store(at, c, part[tid]);
     }
   };
+  auto store = [&](int s) {
+    if (tid < NB && first(s) + tid < n) g.b[first(s) + tid] = part[tid];
+  };
 
-  if (rank == 0) {
-    prefetch(0);
-    solve(0);
-  }
+  cluster_arrive();  // every CTA has started: its shared memory may be written
+  stage_block(rank);
+  if (rank == 1 % C && nblk > 1) load_tile(first(1), first(0));
+  cluster_wait();
+  if (rank == 0) solve(0);
   cluster_arrive();
-  if (rank == 1 % C && nblk > 1) {
-    __syncthreads();
-    prefetch(1);
+  if (rank == 0) {
+    store(0);
+    __syncthreads();  // the inverse has been read
+    stage_block(C);
   }
   cluster_wait();
   for (int s = 0; s + 1 < nblk; ++s) {
     const int k0 = first(s);
-    __syncthreads();  // the previous step's reads of xs are done
-    if (tid < NB) xs[tid] = k0 + tid < n ? __ldcg(g.b + k0 + tid) : 0.0;
-    __syncthreads();
-    if ((s + 1) % C == rank) {
+    const bool mine = (s + 1) % C == rank;
+    if (mine) {
       fold((s + 1) / C, first(s + 1), s);
       solve(s + 1);
     }
+    // slot (s + 1) mod 3 held x_{s−2}: a CTA behind this one is folding x_{s−1}
+    // at the latest (it has arrived at the barrier before), so nobody reads it
     cluster_arrive();
+    if (mine) {
+      store(s + 1);
+      __syncthreads();  // the inverse has been read
+      stage_block(s + 1 + C);
+    }
     for (int t = s + 2 + (rank - (s + 2) % C + C) % C; t < nblk; t += C) {
       load_tile(first(t), k0);
       fold(t / C, first(t), s);
     }
-    if ((s + 2) % C == rank && s + 2 < nblk) {
-      if (C == 1) __syncthreads();  // this CTA also used the inverse at this step
-      prefetch(s + 2);
-    }
+    if ((s + 2) % C == rank && s + 2 < nblk) load_tile(first(s + 2), first(s + 1));
     cluster_wait();
   }
 }
