@@ -24,7 +24,7 @@
 // skipped and warps whose block is wholly above it only help load.
 // kmode: CG_FULL kb = 0; CG_FROM_ROW kb = the tile's first row (opA(i,k) = 0
 // for k < i); CG_FROM_COL kb = the tile's first column (opB(k,j) = 0 for
-// k < j); CG_TO_ROW the k range ends at the tile's last row (opA(i,k) = 0 for
+// k < j; each warp starts at its own first column); CG_TO_ROW the k range ends at the tile's last row (opA(i,k) = 0 for
 // k > i); CG_TO_COL each warp's ends at its own last column (opB(k,j) = 0 for
 // k > j; a scheduler's warps hold different columns, so it saves DMMA time where
 // one tile spans the triangle).  A tile reads all its inputs before it writes C,
@@ -240,6 +240,7 @@ __device__ void cta_gemm_tile(int M, int N, int K, const double* A, long long ld
 #pragma unroll
         for (int kk = 0; kk < CG_K; kk += 4) {
           if (kmode == CG_TO_COL && c * CG_K + kk >= klim) break;
+          if (kmode == CG_FROM_COL && c * CG_K + kk + 4 <= wn * WN) continue;  // k below the warp's columns
           double a[MI][2], b[NJ];
 #pragma unroll
           for (int mi = 0; mi < MI; ++mi) {
