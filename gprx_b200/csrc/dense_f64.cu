@@ -831,7 +831,8 @@ cudaError_t gemv_t(const double* M, long long ld, int nrows, int ncols, bool low
 
 template <bool BLOCK>
 __global__ void __launch_bounds__(256) col_sumsq_kernel(const double* M, long long ld, int nrows, int ncols,
-                                                        const double* w, double* out, const DevStatus* st) {
+                                                        const double* w, double* out, VarianceOf var,
+                                                        const DevStatus* st) {
   constexpr int G = BLOCK ? 256 : 32;
   if (dev_failed(st)) return;
   const int c = (blockIdx.x * 256 + threadIdx.x) / G, t = threadIdx.x % G;
@@ -843,14 +844,17 @@ __global__ void __launch_bounds__(256) col_sumsq_kernel(const double* M, long lo
     acc = w ? fma(v, v / w[i], acc) : fma(v, v, acc);
   }
   acc = column_sum<BLOCK>(acc);
-  if (t == 0) out[c] = acc;
+  if (t != 0) return;
+  const double lat = var.kss - acc;
+  out[c] = var.on ? (lat < 0.0 ? 0.0 : lat) + var.add : acc;  // a NaN stays one
 }
 
 cudaError_t col_sumsq(const double* M, long long ld, int nrows, int ncols, const double* w, double* out,
-                      DevStatus* st, cudaStream_t s, bool block) {
+                      DevStatus* st, cudaStream_t s, bool block, VarianceOf var) {
   if (ncols <= 0) return cudaSuccess;
-  if (block) GPRX_LAUNCH(col_sumsq_kernel<true>, ncols, 256, 0, s, M, ld, nrows, ncols, w, out, st);
-  else GPRX_LAUNCH(col_sumsq_kernel<false>, ceil_div((long long)ncols * 32, 256), 256, 0, s, M, ld, nrows, ncols, w, out, st);
+  const int grid = block ? ncols : ceil_div((long long)ncols * 32, 256);
+  if (block) GPRX_LAUNCH(col_sumsq_kernel<true>, grid, 256, 0, s, M, ld, nrows, ncols, w, out, var, st);
+  else GPRX_LAUNCH(col_sumsq_kernel<false>, grid, 256, 0, s, M, ld, nrows, ncols, w, out, var, st);
   return cudaGetLastError();
 }
 

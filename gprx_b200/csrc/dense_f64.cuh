@@ -101,8 +101,13 @@ cudaError_t trmv_lower(const double* X, long long ld, int n, const double* y, do
 cudaError_t gemv_t(const double* M, long long ld, int nrows, int ncols, bool lower, const double* v, double* out,
                    DevStatus* st, cudaStream_t s, bool block = false);
 // out_j = Σ_i M(i,j)² (/ w_i when w != nullptr) for j < ncols.
+// VarianceOf (on): the latent variance max(0, kss − sum) plus `add` instead.
+struct VarianceOf {
+  bool on = false;
+  double kss = 0.0, add = 0.0;
+};
 cudaError_t col_sumsq(const double* M, long long ld, int nrows, int ncols, const double* w, double* out,
-                      DevStatus* st, cudaStream_t s, bool block = false);
+                      DevStatus* st, cudaStream_t s, bool block = false, VarianceOf var = {});
 
 // out = Σ_i a_i b_i (single block, deterministic).
 cudaError_t dot_dev(const double* a, const double* b, int n, double* out, DevStatus* st, cudaStream_t s);

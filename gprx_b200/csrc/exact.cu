@@ -520,17 +520,6 @@ gprx_status ExactState::nlml(double* out) {
   return GPRX_OK;
 }
 
-// var = max(0, k** − quad) (+ σn² for observation variance); shared.rs:792-806
-__global__ void finish_var_kernel(const double* quad, int q, double kss, double noise, int kind, double* var,
-                                  const DevStatus* st) {
-  if (dev_failed(st)) return;
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= q) return;
-  double lat = kss - quad[j];
-  if (lat < 0.0) lat = 0.0;
-  var[j] = kind == GPRX_VARIANCE_OBSERVATION ? lat + noise : lat;
-}
-
 __global__ void extract_diag_kernel(const double* A, long long ld, int n, double* out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = A[i + (long long)i * ld];
@@ -868,18 +857,16 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
     double* xq = qx.p;                  // qc × d
     double* mdev = qx.p + (size_t)qc_max * d;
     double* vdev = mdev + qc_max;
-    double* quad = vdev + qc_max;
     GPRX_CUDA_TRY(cudaMemcpy2DAsync(xq, sizeof(double) * qc, xs + c0, sizeof(double) * q, sizeof(double) * qc, d,
                                     cudaMemcpyHostToDevice, stream));
     GPRX_CUDA_TRY(fill_cross(kern, x.p, cap, n, xq, qc, qc, qbuf.p, ld, status.p, stream));
     GPRX_CUDA_TRY(gemv_t(qbuf.p, ld, n, qc, false, alpha.p, mdev, status.p, stream, cls == SOLVE_FEW));
     GPRX_CUDA_TRY(trsm_lower(cls, A.p, ld, n, linv.p, qbuf.p, ld, qc, status.p, stream));
-    GPRX_CUDA_TRY(col_sumsq(qbuf.p, ld, n, qc, online ? tmpv.p : nullptr, quad, status.p, stream,
-                            cls == SOLVE_FEW));
-    finish_var_kernel<<<ceil_div(qc, 256), 256, 0, stream>>>(quad, qc, kss, noise(), kind, vdev, status.p);
-    count_launch();
-    GPRX_CUDA_TRY(cudaMemcpyAsync(hm, mdev, sizeof(double) * qc, cudaMemcpyDeviceToHost, stream));
-    GPRX_CUDA_TRY(cudaMemcpyAsync(hm + qc_max, vdev, sizeof(double) * qc, cudaMemcpyDeviceToHost, stream));
+    // var = max(0, k** − ‖V‖²) (+ σn² for observation variance); shared.rs:792-806
+    GPRX_CUDA_TRY(col_sumsq(qbuf.p, ld, n, qc, online ? tmpv.p : nullptr, vdev, status.p, stream, cls == SOLVE_FEW,
+                            VarianceOf{true, kss, kind == GPRX_VARIANCE_OBSERVATION ? noise() : 0.0}));
+    // mean and variance lie one after the other: one copy
+    GPRX_CUDA_TRY(cudaMemcpyAsync(hm, mdev, sizeof(double) * (qc_max + qc), cudaMemcpyDeviceToHost, stream));
     DevStatus ds;
     if ((st = read_status(&ds)) != GPRX_OK) return st;
     if (ds.code != GPRX_OK) return status_to_error(ds, jitter, n, GPRX_STAGE_PREDICT);
