@@ -774,18 +774,19 @@ __global__ void fit_finish_kernel(FitArgs a, double* log_theta_out, FitResult* o
 // ---------------------------------------------------------------------------
 struct BatchState {
   int device = 0;
-  cudaStream_t stream = nullptr;
+  Lane lane;  // first: the buffers' releases wait for it
+  cudaStream_t stream = nullptr;  // lane's main stream
   int nprob = 0, d = 0, p = 0, nmax = 0;
   gprx_options opt{};
   HostKernel kern;
   std::vector<int> n_host;
-  DevBuf<double> x, y, work, theta, nlml, grad, zstart, theta_out;
-  DevBuf<BatchProblem> probs;
-  DevBuf<int> order, status, active;
-  DevBuf<BatchHeader> hdr;
-  DevBuf<ProblemFit> fits;
-  DevBuf<FitResult> results;
-  HostPinned<BatchHeader> hdr_h;
+  DevBuf<double> x{lane}, y{lane}, work{lane}, theta{lane}, nlml{lane}, grad{lane}, zstart{lane}, theta_out{lane};
+  DevBuf<BatchProblem> probs{lane};
+  DevBuf<int> order{lane}, status{lane}, active{lane};
+  DevBuf<BatchHeader> hdr{lane};
+  DevBuf<ProblemFit> fits{lane};
+  DevBuf<FitResult> results{lane};
+  HostPinned<BatchHeader> hdr_h{lane};
   int ctas = 0;
   size_t smem = 0;
   cudaGraphExec_t graph = nullptr;
@@ -799,12 +800,11 @@ struct BatchState {
   int8_t tiles[BATCH_SIZE_CLASSES] = {};
   float tune_ms[BATCH_SIZE_CLASSES][CG_CONFIGS] = {};
   bool tuned = false, tiles_fixed = false;
-  DevBuf<int> tune_order;
+  DevBuf<int> tune_order{lane};
 
   ~BatchState() {
-    if (stream) cudaStreamSynchronize(stream);
+    lane.close();
     if (graph) cudaGraphExecDestroy(graph);
-    stream_release(stream, false, device);
   }
 
   gprx_status create(const double* xh, const double* yh, const uint64_t* ns, uint64_t np, uint64_t dd,
@@ -869,7 +869,8 @@ gprx_status BatchState::create(const double* xh, const double* yh, const uint64_
   p = n_theta;
   device = opt.device;
   GPRX_CUDA_TRY(cudaSetDevice(device));
-  GPRX_CUDA_TRY(stream_acquire(&stream, false));
+  GPRX_CUDA_TRY(lane.open());
+  stream = lane.main();
   int sms = 0;
   GPRX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   smem = batch_smem();

@@ -15,7 +15,6 @@
 #include "dense_f64.cuh"
 #include "emu_gemm.cuh"
 #include "diag_block.cuh"
-#include "pool.h"
 
 namespace gprx {
 
@@ -183,14 +182,10 @@ FactorCtx::~FactorCtx() {
   for (auto e : ev) cudaEventDestroy(e);
   for (auto e : side)
     if (e) cudaEventDestroy(e);
-  stream_release(aux, true, device);
-  stream_release(aux2, true, device);
 }
 
 cudaError_t FactorCtx::ensure(int nblk) {
-  if (!aux || !aux2) CK(cudaGetDevice(&device));
-  if (!aux) CK(stream_acquire(&aux, true));
-  if (!aux2) CK(stream_acquire(&aux2, true));
+  CK(lane.open_sides());
   for (auto& e : side)
     if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   while ((int)ev.size() < 3 * nblk + 2) {
@@ -427,12 +422,12 @@ cudaError_t potrf_blocked(double* A, long long ld, int n, double* linv, DevStatu
     return cudaGetLastError();
   }
   CK(ctx->ensure(nblk));
-  cudaStream_t X = ctx->aux;
+  cudaStream_t X = ctx->lane.aux();
   cudaEvent_t* Ep = ctx->ev.data();          // panel k done (on X)
   cudaEvent_t* Es = ctx->ev.data() + nblk;   // trailing update of step k done (on s)
   cudaEvent_t* Ec = ctx->ev.data() + 2 * nblk + 2;  // column update's lower rows of step k done (on aux2)
   cudaEvent_t Ein = ctx->ev[2 * nblk];
-  cudaStream_t X2 = ctx->aux2;
+  cudaStream_t X2 = ctx->lane.aux2();
   CK(cudaEventRecord(Ein, s));
   CK(cudaStreamWaitEvent(X, Ein, 0));
   CK(diag_and_panel(A, ld, n, 0, linv, st, X));

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "gemm_f64.cuh"
+#include "pool.h"
 
 namespace gprx {
 
@@ -25,11 +26,12 @@ GemmParams gemm_params(int M, int N, int K, const double* A, long long lda, cons
 // block (concurrent with the diagonal block).  After the factor, aux is free
 // for work beside the inverse's products (side: events for that).
 struct FactorCtx {
-  int device = -1;
-  cudaStream_t aux = nullptr;
-  cudaStream_t aux2 = nullptr;
+  Lane& lane;  // of the handle: aux and aux2 are its side streams
   std::vector<cudaEvent_t> ev;
   cudaEvent_t side[4] = {nullptr, nullptr, nullptr, nullptr};
+  explicit FactorCtx(Lane& l) : lane(l) {}
+  FactorCtx(const FactorCtx&) = delete;
+  FactorCtx& operator=(const FactorCtx&) = delete;
   ~FactorCtx();
   cudaError_t ensure(int nblk);
 };

@@ -23,10 +23,9 @@
 namespace gprx {
 
 ExactState::~ExactState() {
-  if (stream) cudaStreamSynchronize(stream);
+  lane.close();
   for (auto& e : ev)
     if (e) cudaEventDestroy(e);
-  stream_release(stream, false, device);
 }
 
 static bool in_default_interval(double log_v) {
@@ -60,7 +59,8 @@ gprx_status ExactState::create(const double* xh, uint64_t nn, uint64_t dd, const
   ld = round_ld(cap);
   device = opt.device;
   GPRX_CUDA_TRY(cudaSetDevice(device));
-  GPRX_CUDA_TRY(stream_acquire(&stream, false));
+  GPRX_CUDA_TRY(lane.open());
+  stream = lane.main();
   for (auto& e : ev) GPRX_CUDA_TRY(cudaEventCreate(&e));
   int nblk = ceil_div(cap, NB);
   if (x.alloc((size_t)cap * d) != cudaSuccess || y.alloc(cap) != cudaSuccess ||
@@ -258,7 +258,7 @@ gprx_status ExactState::eval(const double* params, double* nlml_out, double* gra
       // the log-det and α = Xᵀ (X y) run on the side stream beside K⁻¹ = XᵀX:
       // one-CTA and memory-bound kernels next to the products (35 µs off the
       // stream at n = 1537)
-      cudaStream_t side = fctx.aux;
+      cudaStream_t side = lane.aux();
       GPRX_CUDA_TRY(cudaEventRecord(fctx.side[0], stream));
       GPRX_CUDA_TRY(cudaStreamWaitEvent(side, fctx.side[0], 0));
       GPRX_CUDA_TRY(logdet_diag(A.p, ld, n, false, res.p + 0, status.p, side));
@@ -430,7 +430,7 @@ gprx_status ExactState::hessian(const double* params, double* out, double* nlml_
   };
   // v_i on the side stream beside the products: memory-bound kernels of 15 and
   // 18 µs at n = 2048 that would wait in line with them
-  cudaStream_t side = fctx.aux;
+  cudaStream_t side = lane.aux();
   for (int i = 0; i < pk; ++i) {
     if (i > 0) GPRX_CUDA_TRY(cudaStreamWaitEvent(stream, fctx.side[1], 0));  // the side stream has read the last D
     GPRX_CUDA_TRY(fill_deriv(kern, hm, i, x.p, cap, n, D, ld, stream));

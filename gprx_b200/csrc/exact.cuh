@@ -33,7 +33,8 @@ gprx_status draw_posterior(const double* cov, int q, const double* mean_host, ui
 
 struct ExactState {
   int device = 0;
-  cudaStream_t stream = nullptr;
+  Lane lane;  // first: the buffers' releases wait for it
+  cudaStream_t stream = nullptr;  // lane's main stream
   int n = 0, d = 0;
   long long ld = 0;        // leading dimension of the n×n buffers
   int cap = 0;             // online capacity (rows/cols the buffers hold)
@@ -42,29 +43,29 @@ struct ExactState {
   double log_noise = 0.0;
   std::vector<double> y_host;  // y in buffer order (online compaction)
 
-  DevBuf<double> x;        // cap×d (column-major, ld = cap)
-  DevBuf<double> y;        // cap
-  DevBuf<double> A;        // ld×cap: K → L (→ K⁻¹ after a gradient; → LDLT online)
-  DevBuf<double> Xinv;     // ld×cap: L⁻¹ (gradient path; strict upper triangle kept zero)
-  DevBuf<double> scratch;  // ceil(n/2)² doubles for the recursive triangular inverse
-  DevBuf<double> linv;     // diagonal-block inverses
-  DevBuf<double> alpha, z, tmpv;
-  DevBuf<double> partials;
-  DevBuf<int> slot_param;
-  DevBuf<double> res;      // [0] logdet, [1] yᵀα, [2..] grad
-  DevBuf<DevStatus> status;
-  FactorCtx fctx;          // side stream + events of the look-ahead factor
-  HostPinned<double> res_h;
-  HostPinned<DevStatus> status_h;
-  DevBuf<double> qbuf, qx;  // predict scratch
-  HostPinned<double> pred_h;
-  DevBuf<unsigned char> group_dev;       // grouped-predict staging (this handle leads the group)
-  HostPinned<unsigned char> group_host;
+  DevBuf<double> x{lane};        // cap×d (column-major, ld = cap)
+  DevBuf<double> y{lane};        // cap
+  DevBuf<double> A{lane};        // ld×cap: K → L (→ K⁻¹ after a gradient; → LDLT online)
+  DevBuf<double> Xinv{lane};     // ld×cap: L⁻¹ (gradient path; strict upper triangle kept zero)
+  DevBuf<double> scratch{lane};  // ceil(n/2)² doubles for the recursive triangular inverse
+  DevBuf<double> linv{lane};     // diagonal-block inverses
+  DevBuf<double> alpha{lane}, z{lane}, tmpv{lane};
+  DevBuf<double> partials{lane};
+  DevBuf<int> slot_param{lane};
+  DevBuf<double> res{lane};      // [0] logdet, [1] yᵀα, [2..] grad
+  DevBuf<DevStatus> status{lane};
+  FactorCtx fctx{lane};          // events of the look-ahead factor (on the lane's side streams)
+  HostPinned<double> res_h{lane};
+  HostPinned<DevStatus> status_h{lane};
+  DevBuf<double> qbuf{lane}, qx{lane};  // predict scratch
+  HostPinned<double> pred_h{lane};
+  DevBuf<unsigned char> group_dev{lane};       // grouped-predict staging (this handle leads the group)
+  HostPinned<unsigned char> group_host{lane};
   // mixed precision: the inverse's products emulated on the int8 tensor cores
-  DevBuf<int8_t> emu_sa, emu_sb;
-  DevBuf<int> emu_ea, emu_eb, emu_err;
-  DevBuf<unsigned long long> emu_ma, emu_mb;
-  HostPinned<int> emu_err_h;
+  DevBuf<int8_t> emu_sa{lane}, emu_sb{lane};
+  DevBuf<int> emu_ea{lane}, emu_eb{lane}, emu_err{lane};
+  DevBuf<unsigned long long> emu_ma{lane}, emu_mb{lane};
+  HostPinned<int> emu_err_h{lane};
 
   bool factor_ok = false;   // A holds L (LLT) of the current θ
   bool alpha_ok = false;
@@ -110,12 +111,12 @@ struct ExactState {
   gprx_status nlml(double* out);
   // Hessian of the NLML at params (row-major p × p); the value and the
   // gradient of the same evaluation when nlml_out / grad_out are given
-  DevBuf<double> hs_s, hs_p, hs_d, hs_v, hs_part, hs_res;
-  HostPinned<double> hs_res_h;
+  DevBuf<double> hs_s{lane}, hs_p{lane}, hs_d{lane}, hs_v{lane}, hs_part{lane}, hs_res{lane};
+  HostPinned<double> hs_res_h{lane};
   gprx_status hessian(const double* params, double* out, double* nlml_out = nullptr, double* grad_out = nullptr);
   gprx_status predict(const double* xs, uint64_t q, int kind, double* mean, double* var);
   // leave-one-out, query covariance and posterior draws from the resident factor
-  DevBuf<double> covbuf, covl, covlinv, zbuf;
+  DevBuf<double> covbuf{lane}, covl{lane}, covlinv{lane}, zbuf{lane};
   gprx_status ready_for_query();
   gprx_status loo(int kind, double* mean, double* var);
   gprx_status covariance_dev(const double* xs, uint64_t q, int kind, double* mean_host);
@@ -135,9 +136,9 @@ struct ExactState {
   // plain LLT: afterwards A is the LDLT at the model's θ again, and a failed
   // op leaves the LDLT, α and the jitter as they were
   // (with_llt_view, src/gpr/online.rs:1151-1185).
-  DevBuf<double> ldlt_keep, alpha_keep;
-  DevBuf<double> spare_A, spare_x, spare_y;  // a delete writes here, then swaps
-  DevBuf<double> r1;                         // its vectors: p, β, new D, per-block sums
+  DevBuf<double> ldlt_keep{lane}, alpha_keep{lane};
+  DevBuf<double> spare_A{lane}, spare_x{lane}, spare_y{lane};  // a delete writes here, then swaps
+  DevBuf<double> r1{lane};                         // its vectors: p, β, new D, per-block sums
   gprx_status with_llt_view(const std::function<gprx_status()>& op);
   gprx_status online_insert(const double* xnew, double ynew, uint64_t* id);
   gprx_status online_delete(uint64_t id);

@@ -202,7 +202,7 @@ gprx_status ExactState::grow(int needed) {
   if (needed <= cap) return GPRX_OK;
   int new_cap = std::max(needed, std::max(cap, 1) * 2);
   long long new_ld = round_ld(new_cap);
-  DevBuf<double> nA, nx, ny;
+  DevBuf<double> nA{lane}, nx{lane}, ny{lane};
   if (nA.alloc((size_t)new_ld * new_cap) != cudaSuccess || nx.alloc((size_t)new_cap * d) != cudaSuccess ||
       ny.alloc(new_cap) != cudaSuccess)
     return set_error(GPRX_OUT_OF_MEMORY, "online capacity growth");

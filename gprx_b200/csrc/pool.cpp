@@ -8,11 +8,15 @@
 //  * device buffers up to POOL_MAX_BLOCK come from one CUDA memory pool per
 //    device (3 µs).  An allocation is ordered on a private stream that is
 //    drained before the pointer is returned, so any stream may use it at once;
-//    a free first waits for the device, as cudaFree does.  The pool gives
+//    a free first waits for its owner's streams (Lane).  The pool gives
 //    memory above POOL_KEEP back to the driver whenever it is drained, and all
 //    of its unused memory when an allocation fails.
 //  * pinned blocks and idle streams are kept in small bounded lists (PINNED_KEEP
 //    bytes, STREAM_KEEP streams of a kind); what does not fit is freed.
+//
+// Nothing here waits for the whole device: that is an error while any stream is
+// being captured (a batched fit's rounds on another thread, a caller's graph)
+// and ends the capture with an error of its own.
 //
 // Every list is behind one mutex.  Buffers keep their device, so they may be
 // freed with any device current.  The lists live until the process ends.
@@ -98,31 +102,21 @@ cudaError_t device_alloc(void** out, size_t bytes, int* device) {
       stream = d->stream;
     }
   }
-  if (pool && bytes <= POOL_MAX_BLOCK) {
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
-      if (e == cudaSuccess) return cudaStreamSynchronize(stream);
-      (void)cudaGetLastError();
-      *out = nullptr;
-      if (attempt == 0) {
-        cudaDeviceSynchronize();
-        cudaMemPoolTrimTo(pool, 0);
-      }
-    }
-    return e;
-  }
-  e = cudaMalloc(out, bytes);
-  if (e == cudaErrorMemoryAllocation && pool) {
+  const bool pooled = pool && bytes <= POOL_MAX_BLOCK;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    e = pooled ? cudaMallocFromPoolAsync(out, bytes, pool, stream) : cudaMalloc(out, bytes);
+    if (e == cudaSuccess) return pooled ? cudaStreamSynchronize(stream) : e;
     (void)cudaGetLastError();
-    cudaDeviceSynchronize();
+    *out = nullptr;
+    if (e != cudaErrorMemoryAllocation || !pool) break;
+    // what the pool holds unused goes back to the driver
+    cudaStreamSynchronize(stream);
     cudaMemPoolTrimTo(pool, 0);
-    e = cudaMalloc(out, bytes);
   }
-  if (e != cudaSuccess) *out = nullptr;
   return e;
 }
 
-void device_free(void* ptr, size_t bytes, int device) {
+void device_free(void* ptr, size_t bytes, int device, const Lane& lane) {
   if (!ptr) return;
   cudaStream_t stream = nullptr;
   {
@@ -130,17 +124,12 @@ void device_free(void* ptr, size_t bytes, int device) {
     std::lock_guard<std::mutex> lock(p.mu);
     if (DevicePool* d = device_pool(p, device)) stream = d->stream;
   }
-  if (!stream || bytes > POOL_MAX_BLOCK) {
-    cudaFree(ptr);
-    return;
-  }
-  int was = device;
-  cudaGetDevice(&was);
-  if (was != device) cudaSetDevice(device);
-  // a wait that was refused (a capture elsewhere) leaves it to cudaFree's own
-  if (cudaDeviceSynchronize() == cudaSuccess) cudaFreeAsync(ptr, stream);
-  else cudaFree(ptr);
-  if (was != device) cudaSetDevice(was);
+  const bool idle = lane.drain();
+  cudaError_t e = cudaSuccess;
+  if (!stream || bytes > POOL_MAX_BLOCK) e = cudaFree(ptr);
+  else if (idle) e = cudaFreeAsync(ptr, stream);
+  // else: work that may use it could not be waited for, so nobody else gets it
+  if (e != cudaSuccess) (void)cudaGetLastError();
 }
 
 cudaError_t pinned_alloc(void** out, size_t bytes) {
@@ -161,11 +150,10 @@ cudaError_t pinned_alloc(void** out, size_t bytes) {
   return cudaMallocHost(out, c);
 }
 
-void pinned_free(void* ptr, size_t bytes) {
+void pinned_free(void* ptr, size_t bytes, const Lane& lane) {
   if (!ptr) return;
   const size_t c = pinned_class(bytes);
-  if (c <= PINNED_MAX_BLOCK) {
-    cudaDeviceSynchronize();  // cudaFreeHost's wait: no copy into the block is in flight
+  if (c <= PINNED_MAX_BLOCK && lane.drain()) {  // no copy into the block is in flight
     Pools& p = pools();
     std::lock_guard<std::mutex> lock(p.mu);
     if (p.pinned_bytes + c <= PINNED_KEEP) {
@@ -174,10 +162,11 @@ void pinned_free(void* ptr, size_t bytes) {
       return;
     }
   }
-  cudaFreeHost(ptr);
+  if (cudaFreeHost(ptr) != cudaSuccess) (void)cudaGetLastError();
 }
 
-cudaError_t stream_acquire(cudaStream_t* out, bool high) {
+// A non-blocking stream of the current device, normal or highest priority.
+static cudaError_t stream_acquire(cudaStream_t* out, bool high) {
   *out = nullptr;
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
@@ -198,9 +187,9 @@ cudaError_t stream_acquire(cudaStream_t* out, bool high) {
   return cudaStreamCreateWithPriority(out, cudaStreamNonBlocking, hi);
 }
 
-void stream_release(cudaStream_t s, bool high, int device) {
-  if (!s) return;
-  if (cudaStreamSynchronize(s) == cudaSuccess) {
+// Back to the list; one that was not drained is given up.
+static void stream_release(cudaStream_t s, bool high, int device, bool drained) {
+  if (drained) {
     Pools& p = pools();
     std::lock_guard<std::mutex> lock(p.mu);
     auto& list = p.dev[device].idle[high ? 1 : 0];
@@ -209,7 +198,40 @@ void stream_release(cudaStream_t s, bool high, int device) {
       return;
     }
   }
-  cudaStreamDestroy(s);
+  if (cudaStreamDestroy(s) != cudaSuccess) (void)cudaGetLastError();
+}
+
+cudaError_t Lane::open() {
+  if (s_[0]) return cudaSuccess;
+  cudaError_t e = cudaGetDevice(&device_);
+  return e != cudaSuccess ? e : stream_acquire(&s_[0], false);
+}
+
+cudaError_t Lane::open_sides() {
+  for (int i = 1; i < 3; ++i) {
+    if (s_[i]) continue;
+    const cudaError_t e = stream_acquire(&s_[i], true);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+bool Lane::drain() const {
+  bool ok = true;
+  for (cudaStream_t s : s_)
+    if (s && cudaStreamSynchronize(s) != cudaSuccess) {
+      (void)cudaGetLastError();
+      ok = false;
+    }
+  return ok;
+}
+
+void Lane::close() {
+  const bool drained = drain();
+  for (int i = 0; i < 3; ++i) {
+    if (s_[i]) stream_release(s_[i], i > 0, device_, drained);
+    s_[i] = nullptr;
+  }
 }
 
 }  // namespace gprx

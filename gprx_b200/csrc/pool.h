@@ -7,18 +7,37 @@
 
 namespace gprx {
 
+// The streams of one owner (a handle).  All work on the owner's buffers is
+// ordered by them, so a buffer's release waits for them and for nothing else:
+// no wait on the device, which a capture on any other stream would forbid.
+class Lane {
+ public:
+  Lane() = default;
+  Lane(const Lane&) = delete;
+  Lane& operator=(const Lane&) = delete;
+  ~Lane() { close(); }
+  cudaError_t open();        // the main stream, on the current device
+  cudaError_t open_sides();  // two of the highest priority
+  // Waits for every stream; false when one cannot be waited for.
+  bool drain() const;
+  // Drains and gives the streams back; later releases have nothing to wait for.
+  void close();
+  cudaStream_t main() const { return s_[0]; }
+  cudaStream_t aux() const { return s_[1]; }
+  cudaStream_t aux2() const { return s_[2]; }
+
+ private:
+  int device_ = 0;
+  cudaStream_t s_[3] = {nullptr, nullptr, nullptr};
+};
+
 // Device memory on the current device (*device receives it); usable from any
-// stream on return.  device_free waits for the device first.
+// stream on return.
 cudaError_t device_alloc(void** out, size_t bytes, int* device);
-void device_free(void* ptr, size_t bytes, int device);
+void device_free(void* ptr, size_t bytes, int device, const Lane& lane);
 
 // Pinned host memory; pinned_free takes the size asked for.
 cudaError_t pinned_alloc(void** out, size_t bytes);
-void pinned_free(void* ptr, size_t bytes);
-
-// Non-blocking streams of the current device, normal or highest priority;
-// stream_release drains the stream.
-cudaError_t stream_acquire(cudaStream_t* out, bool high);
-void stream_release(cudaStream_t s, bool high, int device);
+void pinned_free(void* ptr, size_t bytes, const Lane& lane);
 
 }  // namespace gprx

@@ -253,6 +253,12 @@ static gprx_status predict_group(gprx_exact* const* hs, uint64_t k, const double
     qo += q;
   }
   gprx_status st;
+  // the other models' buffers are read on this stream: an early return must
+  // not leave it running, their releases wait for their own streams only
+  struct Drain {
+    const Lane& lane;
+    ~Drain() { lane.drain(); }
+  } drain{s0.lane};
   if ((st = s0.reset_status()) != GPRX_OK) return st;
   GPRX_CUDA_TRY(cudaMemcpyAsync(db, hb, up, cudaMemcpyHostToDevice, s0.stream));
   const GroupReq* rq_d = reinterpret_cast<const GroupReq*>(db);

@@ -73,10 +73,11 @@ gprx_status gprx_probe_dgemm(int32_t m, int32_t n, int32_t k, int32_t trans_a, i
   if (m <= 0 || n <= 0 || k <= 0 || reps <= 0 || !ms_per_launch) return set_error(GPRX_INVALID_ARGUMENT, "sizes");
   long long lda = trans_a ? k : m, ldb = trans_b ? n : k;
   size_t sa = (size_t)lda * (trans_a ? m : k), sb = (size_t)ldb * (trans_b ? k : n), sc = (size_t)m * n;
-  DevBuf<double> A, B, Cm;
+  Lane lane;
+  GPRX_CUDA_TRY(lane.open());
+  const cudaStream_t s = lane.main();
+  DevBuf<double> A{lane}, B{lane}, Cm{lane};
   if (A.alloc(sa) || B.alloc(sb) || Cm.alloc(sc)) return set_error(GPRX_OUT_OF_MEMORY, "probe buffers");
-  cudaStream_t s;
-  GPRX_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   fill_pattern_kernel<<<1184, 256, 0, s>>>(A.p, (long long)sa, 1u);
   fill_pattern_kernel<<<1184, 256, 0, s>>>(B.p, (long long)sb, 2u);
   GemmParams p = gemm_params(m, n, k, A.p, lda, B.p, ldb, Cm.p, m, 1.0, 0.0, nullptr);
@@ -92,7 +93,6 @@ gprx_status gprx_probe_dgemm(int32_t m, int32_t n, int32_t k, int32_t trans_a, i
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaStreamDestroy(s);
   if (e != cudaSuccess) return set_cuda_error(e, "probe dgemm");
   if (e2 != cudaSuccess) return set_cuda_error(e2, "probe dgemm sync");
   *ms_per_launch = ms / reps;
@@ -105,18 +105,19 @@ gprx_status gprx_probe_dgemm(int32_t m, int32_t n, int32_t k, int32_t trans_a, i
 gprx_status gprx_probe_potrf(int32_t n, int32_t reps, double* ms_per_factor) {
   if (n <= 0 || reps <= 0 || !ms_per_factor) return set_error(GPRX_INVALID_ARGUMENT, "sizes");
   long long ld = round_ld(n);
-  DevBuf<double> A, linv;
-  DevBuf<DevStatus> st;
+  Lane lane;
+  GPRX_CUDA_TRY(lane.open());
+  const cudaStream_t s = lane.main();
+  DevBuf<double> A{lane}, linv{lane};
+  DevBuf<DevStatus> st{lane};
   if (A.alloc((size_t)ld * n) || linv.alloc((size_t)ceil_div(n, NB) * NB * NB) || st.alloc(1))
     return set_error(GPRX_OUT_OF_MEMORY, "probe buffers");
-  cudaStream_t s;
-  GPRX_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   float total = 0.f;
   cudaError_t e = cudaSuccess;
-  FactorCtx ctx;
+  FactorCtx ctx{lane};
   for (int r = 0; r < reps + 1 && e == cudaSuccess; ++r) {
     cudaMemsetAsync(st.p, 0, sizeof(DevStatus), s);
     fill_spd_kernel<<<1184, 256, 0, s>>>(A.p, ld, n);
@@ -132,7 +133,6 @@ gprx_status gprx_probe_potrf(int32_t n, int32_t reps, double* ms_per_factor) {
   cudaMemcpy(&hs, st.p, sizeof(hs), cudaMemcpyDeviceToHost);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaStreamDestroy(s);
   if (e != cudaSuccess) return set_cuda_error(e, "probe potrf");
   if (hs.code != GPRX_OK) return set_error(hs.code, "probe potrf status");
   *ms_per_factor = total / reps;
@@ -145,10 +145,13 @@ gprx_status gprx_probe_potrf(int32_t n, int32_t reps, double* ms_per_factor) {
 gprx_status gprx_probe_emu_gemm(int32_t m, int32_t n, int32_t k, int32_t S, int32_t reps, double* out) {
   if (m <= 0 || n <= 0 || k <= 0 || reps <= 0 || !out || S < 4 || S > EMU_MAX_S)
     return set_error(GPRX_INVALID_ARGUMENT, "sizes");
-  DevBuf<double> A, B, Aa, Ba, C, R, Cabs;
-  DevBuf<int8_t> sa, sb;
-  DevBuf<int> ea, eb, err;
-  DevBuf<unsigned long long> mx, rma, rmb;
+  Lane lane;
+  GPRX_CUDA_TRY(lane.open());
+  const cudaStream_t s = lane.main();
+  DevBuf<double> A{lane}, B{lane}, Aa{lane}, Ba{lane}, C{lane}, R{lane}, Cabs{lane};
+  DevBuf<int8_t> sa{lane}, sb{lane};
+  DevBuf<int> ea{lane}, eb{lane}, err{lane};
+  DevBuf<unsigned long long> mx{lane}, rma{lane}, rmb{lane};
   EmuOperand a, b;
   a.R = m; a.K = k; a.S = S; a.Rpad = emu_pad_rows(m); a.Kpad = emu_pad_k(k);
   b.R = n; b.K = k; b.S = S; b.Rpad = emu_pad_rows(n); b.Kpad = emu_pad_k(k);
@@ -159,8 +162,6 @@ gprx_status gprx_probe_emu_gemm(int32_t m, int32_t n, int32_t k, int32_t S, int3
       rmb.alloc(b.Rpad))
     return set_error(GPRX_OUT_OF_MEMORY, "probe buffers");
   a.slices = sa.p; a.exps = ea.p; a.rmax = rma.p; b.slices = sb.p; b.exps = eb.p; b.rmax = rmb.p;
-  cudaStream_t s;
-  GPRX_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   fill_pattern_kernel<<<1184, 256, 0, s>>>(A.p, (long long)sza, 3u);
   fill_pattern_kernel<<<1184, 256, 0, s>>>(B.p, (long long)szb, 4u);
   scale_rows_kernel<<<1184, 256, 0, s>>>(A.p, m, m, k);
@@ -216,7 +217,6 @@ gprx_status gprx_probe_emu_gemm(int32_t m, int32_t n, int32_t k, int32_t S, int3
   cudaMemcpy(&hm, mx.p, sizeof(hm), cudaMemcpyDeviceToHost);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaStreamDestroy(s);
   if (e != cudaSuccess) return set_cuda_error(e, "probe emu gemm");
   if (e2 != cudaSuccess) return set_cuda_error(e2, "probe emu gemm sync");
   if (herr) return set_error(GPRX_TIMEOUT, "emulated GEMM: a bounded wait ran out");

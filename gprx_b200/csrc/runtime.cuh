@@ -23,13 +23,14 @@ gprx_status set_cholesky_error(double jitter, uint64_t size, int stage);
     if (e_ != cudaSuccess) return ::gprx::set_cuda_error(e_, #expr); \
   } while (0)
 
-// Owning device buffer.
+// Owning device buffer of the owner with these streams.
 template <typename T>
 struct DevBuf {
+  const Lane& lane;
   T* p = nullptr;
   size_t n = 0;
   int device = 0;
-  DevBuf() = default;
+  explicit DevBuf(const Lane& l) : lane(l) {}
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { reset(); }
@@ -47,7 +48,7 @@ struct DevBuf {
   // grows (never shrinks); contents are not kept
   cudaError_t ensure(size_t count) { return count <= n ? cudaSuccess : alloc(count); }
   void reset() {
-    device_free(p, n * sizeof(T), device);
+    device_free(p, n * sizeof(T), device, lane);
     p = nullptr;
     n = 0;
   }
@@ -56,8 +57,12 @@ struct DevBuf {
 // Pinned host scratch.
 template <typename T>
 struct HostPinned {
+  const Lane& lane;
   T* p = nullptr;
   size_t n = 0;
+  explicit HostPinned(const Lane& l) : lane(l) {}
+  HostPinned(const HostPinned&) = delete;
+  HostPinned& operator=(const HostPinned&) = delete;
   ~HostPinned() { reset(); }
   cudaError_t ensure(size_t count) {
     if (count <= n) return cudaSuccess;
@@ -67,7 +72,7 @@ struct HostPinned {
     return e;
   }
   void reset() {
-    pinned_free(p, n * sizeof(T));
+    pinned_free(p, n * sizeof(T), lane);
     p = nullptr;
     n = 0;
   }

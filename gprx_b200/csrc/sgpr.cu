@@ -308,33 +308,36 @@ static int grid_for(long long work, int per) {
 // ---------------------------------------------------------------------------
 struct SgprState {
   int device = 0;
-  cudaStream_t stream = nullptr;
+  Lane lane;  // first: the buffers' releases wait for it
+  cudaStream_t stream = nullptr;  // lane's main stream
   gprx_options opt{};
   HostKernel kern;
   double log_noise = 0.0;
   long long n = 0, cap = 0;
   int m = 0, d = 0;
   long long ldm = 0;
-  DevBuf<double> x, y, z, Lmm, linv_mm, Amat, Bl, linv_B, w, ay, G, H, Wm, Xb, Xt, splitbuf, partials, res, vtmp,
-      qbuf, qbuf2, qx, Btrial, covbuf, covl, covlinv, zbuf, border;
-  DevBuf<int> slot_param;
-  DevBuf<DevStatus> status;
+  DevBuf<double> x{lane}, y{lane}, z{lane}, Lmm{lane}, linv_mm{lane}, Amat{lane}, Bl{lane}, linv_B{lane}, w{lane},
+      ay{lane}, G{lane}, H{lane}, Wm{lane}, Xb{lane}, Xt{lane}, splitbuf{lane}, partials{lane}, res{lane}, vtmp{lane},
+      qbuf{lane}, qbuf2{lane}, qx{lane}, Btrial{lane}, covbuf{lane}, covl{lane}, covlinv{lane}, zbuf{lane},
+      border{lane};
+  DevBuf<int> slot_param{lane};
+  DevBuf<DevStatus> status{lane};
   // mixed precision: the two m×m Gram products over n (B = A Aᵀ and H = G Aᵀ)
   // emulated on the int8 tensor cores, split over K across CTAs
-  DevBuf<int8_t> emu_sa, emu_sb;
-  DevBuf<double> emu_part;
-  DevBuf<int> emu_ea, emu_eb, emu_err;
-  DevBuf<unsigned long long> emu_ma, emu_mb;
-  HostPinned<int> emu_err_h;
+  DevBuf<int8_t> emu_sa{lane}, emu_sb{lane};
+  DevBuf<double> emu_part{lane};
+  DevBuf<int> emu_ea{lane}, emu_eb{lane}, emu_err{lane};
+  DevBuf<unsigned long long> emu_ma{lane}, emu_mb{lane};
+  HostPinned<int> emu_err_h{lane};
   static constexpr long long EMU_MIN_N = 16384;  // smallest n that uses the emulated products
   static constexpr int EMU_S = 7;                // int8 digits per entry
   static constexpr int EMU_PART_K = 32768;       // K of one split-K part: K·S·2^12 < 2^31 keeps its int32 sums exact
   static constexpr int EMU_GROUP = 8 * EMU_PART_K;  // columns of n sliced at a time (8 parts in flight)
   bool use_emu() const { return opt.precision == GPRX_PRECISION_MIXED && n >= EMU_MIN_N; }
   gprx_status ensure_emu(EmuWork& w);
-  HostPinned<double> res_h;
-  HostPinned<DevStatus> status_h;
-  FactorCtx fctx;
+  HostPinned<double> res_h{lane};
+  HostPinned<DevStatus> status_h{lane};
+  FactorCtx fctx{lane};
   // host scalars of the assembly
   // trace_sum = Σ_c (k(x_c, x_c) − ‖a_c‖²), the numerator of the VFE trace term
   double trace_sum = 0.0, y2 = 0.0, kmm_jitter = 0.0, pivot_ratio = 1.0;
@@ -347,10 +350,9 @@ struct SgprState {
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
 
   ~SgprState() {
-    if (stream) cudaStreamSynchronize(stream);
+    lane.close();
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
-    stream_release(stream, false, device);
   }
 
   double noise() const { return std::exp(log_noise); }
@@ -471,7 +473,8 @@ gprx_status SgprState::create(const double* xh, uint64_t nn, uint64_t dd, const 
   ldm = round_ld(m);
   device = opt.device;
   GPRX_CUDA_TRY(cudaSetDevice(device));
-  GPRX_CUDA_TRY(stream_acquire(&stream, false));
+  GPRX_CUDA_TRY(lane.open());
+  stream = lane.main();
   for (auto& e : ev) GPRX_CUDA_TRY(cudaEventCreate(&e));
   int nblk = ceil_div(m, NB);
   // the m×m factors keep ld columns, the room a bordered inducing insert grows into
@@ -506,7 +509,7 @@ gprx_status SgprState::ensure_points(long long needed) {
   if (needed <= cap && x.p) return GPRX_OK;
   long long new_cap = std::max(needed, std::max(cap, 1LL) * 2);
   if (!x.p) new_cap = needed;
-  DevBuf<double> nx, ny, nA;
+  DevBuf<double> nx{lane}, ny{lane}, nA{lane};
   if (nx.alloc((size_t)new_cap * d) || ny.alloc(new_cap) || nA.alloc((size_t)ldm * new_cap))
     return set_error(GPRX_OUT_OF_MEMORY, "point buffers");
   if (x.p && n > 0) {
@@ -835,7 +838,7 @@ gprx_status SgprState::predict(const double* xs, uint64_t q, int kind, double* m
   if (qbuf.ensure((size_t)ldm * qc_max) || qbuf2.ensure((size_t)ldm * qc_max) ||
       qx.ensure((size_t)qc_max * (d + 4)))
     return set_error(GPRX_OUT_OF_MEMORY, "predict scratch");
-  HostPinned<double> hm;
+  HostPinned<double> hm{lane};
   GPRX_CUDA_TRY(hm.ensure(2 * (size_t)qc_max));
   const double kss = kern.diag_value();
   if ((st = reset_status()) != GPRX_OK) return st;
@@ -1237,7 +1240,7 @@ gprx_status SgprState::set_inducing(const double* zh, uint64_t mm) {
   if ((int)mm != m) {
     int nblk = ceil_div((int)mm, NB);
     // A is re-laid out for the new m (its contents are recomputed below)
-    DevBuf<double> nA;
+    DevBuf<double> nA{lane};
     if (z.alloc((size_t)mm * d) || Lmm.alloc((size_t)new_ldm * new_ldm) || linv_mm.alloc((size_t)nblk * NB * NB) ||
         Bl.alloc((size_t)new_ldm * new_ldm) || linv_B.alloc((size_t)nblk * NB * NB) || w.alloc(new_ldm) ||
         ay.alloc(new_ldm) || vtmp.alloc(new_ldm) || nA.alloc((size_t)new_ldm * std::max(cap, 1LL)))
