@@ -158,7 +158,7 @@ __device__ inline void stage_points(const double* x, int n, int d, int i0, int j
 // lower K + diag_add I into A (ld); returns true when every value is finite
 // (trees of at most NL leaves)
 template <int ARD_D, int NL>
-__device__ bool cta_fill_lower(const KTree& t, const double* x, int n, double* A, long long ld, double diag_add,
+__device__ __noinline__ bool cta_fill_lower(const KTree& t, const double* x, int n, double* A, long long ld, double diag_add,
                                double* smem, int* flag_sh) {
   double* xi = smem;
   double* xj = smem + GPRX_MAX_DIM * FT_B;
@@ -205,7 +205,7 @@ __device__ bool cta_fill_lower(const KTree& t, const double* x, int n, double* A
 // W = ααᵀ − K⁻¹ (K⁻¹ lower in kinv), and Σ W_ii in the last slot (trees of
 // at most NL leaves; the slots of absent leaves are zero).
 template <int ARD_D, int NL>
-__device__ void cta_grad(const KTree& t, const double* x, int n, const double* kinv, long long ld,
+__device__ __noinline__ void cta_grad(const KTree& t, const double* x, int n, const double* kinv, long long ld,
                          const double* alpha, double* smem, double* slots) {
   constexpr int AD = ARD_D > 0 ? ARD_D : 1;
   constexpr int NS = GRAD_SLOTS_LEAF + AD + 1;
@@ -276,20 +276,31 @@ __device__ void cta_grad(const KTree& t, const double* x, int n, const double* k
   __syncthreads();
 }
 
-// the two passes with the leaf bound of the problem's tree: trees of at most two
-// leaves with up to 8 ARD dimensions have their own form (isotropic ones four pairs
-// wide; ARD ones one, two pairs spill: 64 problems of 200 to 256 points 709 µs)
-template <int ARD_D>
-__device__ bool cta_fill_any(const KTree& t, const double* x, int n, double* A, long long ld, double diag_add,
-                             double* smem, int* flag_sh) {
-  if (ARD_D <= 8 && t.n_leaves <= 2) return cta_fill_lower<ARD_D, ARD_D <= 8 ? 2 : KT_MAX_LEAVES>(t, x, n, A, ld, diag_add, smem, flag_sh);
-  return cta_fill_lower<ARD_D, KT_MAX_LEAVES>(t, x, n, A, ld, diag_add, smem, flag_sh);
-}
-template <int ARD_D>
-__device__ void cta_grad_any(const KTree& t, const double* x, int n, const double* kinv, long long ld,
-                             const double* alpha, double* smem, double* slots) {
-  if (ARD_D <= 8 && t.n_leaves <= 2) cta_grad<ARD_D, ARD_D <= 8 ? 2 : KT_MAX_LEAVES>(t, x, n, kinv, ld, alpha, smem, slots);
-  else cta_grad<ARD_D, KT_MAX_LEAVES>(t, x, n, kinv, ld, alpha, smem, slots);
+// The form of the two passes that a tree takes: the width of its ARD leaf and the
+// bound of its leaves (trees of at most two leaves with up to 8 ARD dimensions have
+// their own; isotropic ones four pairs wide, ARD ones one: two pairs spill, 64
+// problems of 200 to 256 points 709 µs).  Every kernel is compiled for one form and
+// calls its two passes out of line: inlined, they and the products push each other's
+// 128 registers into local memory (spill stores of the ARD 8 kernel with both bounds
+// inlined 2780 bytes, one bound 744, one bound called 316).  Measured (µs, both
+// inlined / one inlined / one called): 444 problems of 129 to 256 points, ARD d = 8
+// 2148 / 1728 / 1285, d = 12 3551 / 3551 / 2637, three leaves with ARD d = 4
+// 2082 / 1962 / 1654, isotropic RBF 1004 / 1007 / 984; 296 of 513 to 1024, ARD d = 8
+// 21.2 / 18.4 / 14.3 ms, RBF + periodic 13.6 / 13.7 / 13.5 ms.
+template <int ARD_D, int NL>
+struct Form {
+  static constexpr int ard = ARD_D, nl = NL;
+};
+template <typename F>
+static cudaError_t with_form(const HostKernel& k, F f) {
+  const bool few = k.tree.n_leaves <= 2;
+  switch (k.ard_d) {
+    case 0: return few ? f(Form<0, 2>{}) : f(Form<0, KT_MAX_LEAVES>{});
+    case 4: return few ? f(Form<4, 2>{}) : f(Form<4, KT_MAX_LEAVES>{});
+    case 8: return few ? f(Form<8, 2>{}) : f(Form<8, KT_MAX_LEAVES>{});
+    case 16: return f(Form<16, KT_MAX_LEAVES>{});
+    default: return f(Form<32, KT_MAX_LEAVES>{});
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -357,7 +368,7 @@ inline size_t tile_smem() {
 }
 inline size_t small_smem() { return diag_block_smem() + tile_smem() + 2 * NB_DIAG * sizeof(double); }
 
-template <int ARD_D>
+template <int ARD_D, int NL>
 __device__ __noinline__ int cta_small(const KTree& tree, const double* x, const double* y, int n, double diag_add, double* smem,
                          int* flag_sh, double* red, double* slots, double* alpha, double* logdet, double* quad) {
   double* s = smem;
@@ -368,7 +379,7 @@ __device__ __noinline__ int cta_small(const KTree& tree, const double* x, const 
   double* tiles = av + NB_DIAG;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int np = (n + LF - 1) / LF, npad = np * LF;
-  if (!cta_fill_any<ARD_D>(tree, x, n, s, FLS, diag_add, tiles, flag_sh)) return SMALL_NONFINITE;
+  if (!cta_fill_lower<ARD_D, NL>(tree, x, n, s, FLS, diag_add, tiles, flag_sh)) return SMALL_NONFINITE;
   diag_block_pad(s, n);
   const int f = diag_block_core(nullptr, 0, 0, n, nullptr, false, smem, flag_sh);
   if (f >= 0) return f;
@@ -445,7 +456,7 @@ __device__ __noinline__ int cta_small(const KTree& tree, const double* x, const 
       }
   }
   __syncthreads();
-  cta_grad_any<ARD_D>(tree, x, n, s, FLS, av, tiles, slots);
+  cta_grad<ARD_D, NL>(tree, x, n, s, FLS, av, tiles, slots);
   return -1;
 }
 
@@ -466,7 +477,7 @@ __device__ inline void slots_to_grad(const double* slots, int ns, const int* slo
 // Latency-bound: the pivots' chain and a few passes over one block.  As 12
 // launches (fill, diagonal step, log-det, copy, two products, two vector
 // products, a dot product, K⁻¹, gradient, its sums) n = 64 took 108 µs.
-template <int ARD_D>
+template <int ARD_D, int NL>
 __global__ void __launch_bounds__(BT, 1) small_eval_kernel(const __grid_constant__ KTree tree, const double* x,
                                                            const double* y, int n, double diag_add, double noise,
                                                            int p, const int* slot_param, double* alpha, double* res,
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(BT, 1) small_eval_kernel(const __grid_constant
   __shared__ double slots[64];
   if (dev_failed(st)) return;
   double logdet, quad;
-  const int f = cta_small<ARD_D>(tree, x, y, n, diag_add, smem, &flag_sh, red, slots, alpha, &logdet, &quad);
+  const int f = cta_small<ARD_D, NL>(tree, x, y, n, diag_add, smem, &flag_sh, red, slots, alpha, &logdet, &quad);
   if (threadIdx.x != 0) return;
   if (f != -1) {
     dev_fail(st, f == SMALL_NONFINITE ? GPRX_NONFINITE_KERNEL : GPRX_CHOLESKY_FAILED, f < 0 ? 0 : f);
@@ -488,30 +499,20 @@ __global__ void __launch_bounds__(BT, 1) small_eval_kernel(const __grid_constant
   slots_to_grad(slots, GRAD_SLOTS_LEAF + (ARD_D > 0 ? ARD_D : 1) + 1, slot_param, noise, p, res + 2);
 }
 
-template <int ARD_D>
-static cudaError_t launch_small(const HostKernel& k, const double* x, const double* y, int n, double diag_add,
-                                double noise, const int* slot_param, double* alpha, double* res, DevStatus* st,
-                                cudaStream_t s) {
-  const size_t smem = small_smem();
-  cudaError_t e = cudaFuncSetAttribute(small_eval_kernel<ARD_D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  GPRX_LAUNCH(small_eval_kernel<ARD_D>, 1, BT, smem, s, k.tree, x, y, n, diag_add, noise, k.n_params + 1, slot_param,
-              alpha, res, st);
-  return cudaGetLastError();
-}
-
 cudaError_t small_eval(const HostKernel& k, const double* x, const double* y, int n, double diag_add, double noise,
                        const int* slot_param, double* alpha, double* res, DevStatus* st, cudaStream_t s) {
-  switch (k.ard_d) {
-    case 0: return launch_small<0>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
-    case 4: return launch_small<4>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
-    case 8: return launch_small<8>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
-    case 16: return launch_small<16>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
-    default: return launch_small<32>(k, x, y, n, diag_add, noise, slot_param, alpha, res, st, s);
-  }
+  return with_form(k, [&](auto f) {
+    constexpr int A = decltype(f)::ard, NL = decltype(f)::nl;
+    const size_t smem = small_smem();
+    cudaError_t e = cudaFuncSetAttribute(small_eval_kernel<A, NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    GPRX_LAUNCH((small_eval_kernel<A, NL>), 1, BT, smem, s, k.tree, x, y, n, diag_add, noise, k.n_params + 1,
+                slot_param, alpha, res, st);
+    return cudaGetLastError();
+  });
 }
 
-template <int ARD_D>
+template <int ARD_D, int NL>
 __device__ void cta_eval(const BatchEvalArgs& a, int q, const Work& w, double* smem) {
   __shared__ KTree tree;
   __shared__ int flag_sh, code_sh;
@@ -542,7 +543,7 @@ __device__ void cta_eval(const BatchEvalArgs& a, int q, const Work& w, double* s
     double logdet = 0.0, quad = 0.0;
     for (int attempt = 0; attempt <= a.jit.count; ++attempt) {
       const double j = attempt == 0 ? 0.0 : a.jit.j[attempt - 1];
-      f = cta_small<ARD_D>(tree, P.x, P.y, n, noise + j, smem, &flag_sh, red, slots, w.alpha, &logdet, &quad);
+      f = cta_small<ARD_D, NL>(tree, P.x, P.y, n, noise + j, smem, &flag_sh, red, slots, w.alpha, &logdet, &quad);
       if (f < 0) break;
     }
     if (tid == 0) {
@@ -563,7 +564,7 @@ __device__ void cta_eval(const BatchEvalArgs& a, int q, const Work& w, double* s
   int fail = 0;
   for (int attempt = 0; attempt <= a.jit.count; ++attempt) {
     const double j = attempt == 0 ? 0.0 : a.jit.j[attempt - 1];
-    if (!cta_fill_any<ARD_D>(tree, P.x, n, w.A, ld, noise + j, smem, &flag_sh)) {
+    if (!cta_fill_lower<ARD_D, NL>(tree, P.x, n, w.A, ld, noise + j, smem, &flag_sh)) {
       if (tid == 0) a.status[q] = GPRX_NONFINITE_KERNEL;
       return;
     }
@@ -600,7 +601,7 @@ __device__ void cta_eval(const BatchEvalArgs& a, int q, const Work& w, double* s
   const double quad = block_sum(acc, red);
   // K⁻¹ = Xᵀ X (lower) over L in A
   cta_gemm<true, false>(cfg, n, n, n, w.X, ld, w.X, ld, w.A, ld, 1.0, 0.0, true, CG_FROM_ROW, smem);
-  cta_grad_any<ARD_D>(tree, P.x, n, w.A, ld, w.alpha, smem, slots);
+  cta_grad<ARD_D, NL>(tree, P.x, n, w.A, ld, w.alpha, smem, slots);
   if (tid == 0) {
     constexpr int NS = GRAD_SLOTS_LEAF + (ARD_D > 0 ? ARD_D : 1) + 1;
     const double nl = 0.5 * (quad + logdet + (double)n * log(2.0 * M_PI));
@@ -611,7 +612,7 @@ __device__ void cta_eval(const BatchEvalArgs& a, int q, const Work& w, double* s
   __syncthreads();
 }
 
-template <int ARD_D>
+template <int ARD_D, int NL>
 __global__ void __launch_bounds__(BT, 1) batch_eval_kernel(BatchEvalArgs a) {
   extern __shared__ __align__(16) double smem[];
   __shared__ int pidx;
@@ -624,7 +625,7 @@ __global__ void __launch_bounds__(BT, 1) batch_eval_kernel(BatchEvalArgs a) {
     if (at >= a.nprob) break;
     const int q = a.order[at];
     if (a.active && !a.active[q]) continue;
-    cta_eval<ARD_D>(a, q, w, smem);
+    cta_eval<ARD_D, NL>(a, q, w, smem);
   }
 }
 
@@ -997,32 +998,34 @@ gprx_status BatchState::autotune(const double* log_theta_dev, bool force) {
   return GPRX_OK;
 }
 
-template <int ARD_D>
-static cudaError_t launch_eval_t(const BatchEvalArgs& a, int ctas, size_t smem, cudaStream_t s, bool count) {
-  batch_eval_kernel<ARD_D><<<ctas, BT, smem, s>>>(a);
-  if (count) count_launch();
-  return cudaGetLastError();
+// The batched kernel of a form, launched or with its shared memory allowed (a
+// batch's parameters leave no room for the widest ARD form).
+template <typename FORM>
+static cudaError_t launch_batch_eval(FORM, const BatchEvalArgs& a, int ctas, size_t smem, cudaStream_t s) {
+  if constexpr (FORM::ard > BATCH_MAX_VARS) {
+    return cudaErrorInvalidValue;
+  } else {
+    batch_eval_kernel<FORM::ard, FORM::nl><<<ctas, BT, smem, s>>>(a);
+    return cudaGetLastError();
+  }
+}
+template <typename FORM>
+static cudaError_t allow_batch_eval(FORM) {
+  if constexpr (FORM::ard > BATCH_MAX_VARS) {
+    return cudaErrorInvalidValue;
+  } else {
+    return cudaFuncSetAttribute(batch_eval_kernel<FORM::ard, FORM::nl>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)batch_smem());
+  }
 }
 
 cudaError_t BatchState::launch_eval(const BatchEvalArgs& a, bool count) {
-  switch (kern.ard_d) {
-    case 0: return launch_eval_t<0>(a, ctas, smem, stream, count);
-    case 4: return launch_eval_t<4>(a, ctas, smem, stream, count);
-    case 8: return launch_eval_t<8>(a, ctas, smem, stream, count);
-    case 16: return launch_eval_t<16>(a, ctas, smem, stream, count);
-    default: return launch_eval_t<32>(a, ctas, smem, stream, count);
-  }
+  if (count) count_launch();
+  return with_form(kern, [&](auto f) { return launch_batch_eval(f, a, ctas, smem, stream); });
 }
 
 cudaError_t BatchState::set_eval_attributes() {
-  const int b = (int)smem;
-  switch (kern.ard_d) {
-    case 0: return cudaFuncSetAttribute(batch_eval_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    case 4: return cudaFuncSetAttribute(batch_eval_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    case 8: return cudaFuncSetAttribute(batch_eval_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    case 16: return cudaFuncSetAttribute(batch_eval_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    default: return cudaFuncSetAttribute(batch_eval_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  }
+  return with_form(kern, [](auto f) { return allow_batch_eval(f); });
 }
 
 gprx_status BatchState::eval(const double* log_theta, double* nl, double* g, int32_t* st) {
@@ -1267,13 +1270,10 @@ static gprx_status noalloc_scratch_ptr(int dev, double** out) {
     double* p = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void**)&p, g_noalloc_scratch);
     if (e != cudaSuccess) return set_cuda_error(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
-    const int smem = (int)batch_smem();
-    cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((e = cudaFuncSetAttribute(batch_eval_kernel<0>, a, smem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(batch_eval_kernel<4>, a, smem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(batch_eval_kernel<8>, a, smem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(batch_eval_kernel<16>, a, smem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(batch_eval_kernel<32>, a, smem)) != cudaSuccess)
+    if ((e = allow_batch_eval(Form<0, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<0, KT_MAX_LEAVES>{})) != cudaSuccess ||
+        (e = allow_batch_eval(Form<4, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<4, KT_MAX_LEAVES>{})) != cudaSuccess ||
+        (e = allow_batch_eval(Form<8, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<8, KT_MAX_LEAVES>{})) != cudaSuccess ||
+        (e = allow_batch_eval(Form<16, KT_MAX_LEAVES>{})) != cudaSuccess)
       return set_cuda_error(e, "shared-memory attribute of the evaluation kernel");
     ptrs[dev] = p;
   }
@@ -1355,15 +1355,10 @@ static gprx_status exact_eval_noalloc(const double* x, const double* y, uint64_t
   for (int i = 0; i < 64; ++i) a.slot_param[i] = i < (int)kern.slot_param.size() ? kern.slot_param[i] : -1;
   const size_t smem = batch_smem();
   noalloc_prep_kernel<<<1, NOALLOC_PREP_THREADS, 0, s>>>(scratch, prob, th, (int)p, (int)d);
-  switch (kern.ard_d) {
-    case 0: batch_eval_kernel<0><<<1, BT, smem, s>>>(a); break;
-    case 4: batch_eval_kernel<4><<<1, BT, smem, s>>>(a); break;
-    case 8: batch_eval_kernel<8><<<1, BT, smem, s>>>(a); break;
-    case 16: batch_eval_kernel<16><<<1, BT, smem, s>>>(a); break;
-    default: batch_eval_kernel<32><<<1, BT, smem, s>>>(a); break;
-  }
+  const cudaError_t le = with_form(kern, [&](auto f) { return launch_batch_eval(f, a, 1, smem, s); });
   noalloc_finish_kernel<<<1, 32, 0, s>>>(scratch, (int)p, nlml, grad, status);
   count_launch(3);
+  GPRX_CUDA_TRY(le);
   GPRX_CUDA_TRY(cudaGetLastError());
   return GPRX_OK;
 }
