@@ -8,9 +8,9 @@
 //  * device buffers up to POOL_MAX_BLOCK come from one CUDA memory pool per
 //    device (3 µs).  An allocation is ordered on a private stream that is
 //    drained before the pointer is returned, so any stream may use it at once;
-//    a free first waits for its owner's streams (Lane).  The pool gives
-//    memory above POOL_KEEP back to the driver whenever it is drained, and all
-//    of its unused memory when an allocation fails.
+//    a free first waits for its owner's streams (Lane) and drains it again: then
+//    the pool gives what it holds above POOL_KEEP back to the driver.  All of its
+//    unused memory goes back when an allocation fails.
 //  * pinned blocks and idle streams are kept in small bounded lists (PINNED_KEEP
 //    bytes, STREAM_KEEP streams of a kind); what does not fit is freed.
 //
@@ -127,8 +127,8 @@ void device_free(void* ptr, size_t bytes, int device, const Lane& lane) {
   const bool idle = lane.drain();
   cudaError_t e = cudaSuccess;
   if (!stream || bytes > POOL_MAX_BLOCK) e = cudaFree(ptr);
-  else if (idle) e = cudaFreeAsync(ptr, stream);
-  // else: work that may use it could not be waited for, so nobody else gets it
+  else if (idle && (e = cudaFreeAsync(ptr, stream)) == cudaSuccess) e = cudaStreamSynchronize(stream);  // past POOL_KEEP: to the driver
+  // not idle: work that may use it could not be waited for, so nobody else gets it
   if (e != cudaSuccess) (void)cudaGetLastError();
 }
 
