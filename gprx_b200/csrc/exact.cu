@@ -216,7 +216,7 @@ gprx_status ExactState::eval(const double* params, double* nlml_out, double* gra
   js.insert(js.end(), r.begin(), r.end());
   double last = 0.0;
   const size_t nn = (size_t)ld * cap;
-  const bool small = grad && !keep_inverse && n <= SMALL_EVAL_N && cap == n;
+  const bool small = grad && !keep_inverse && n <= small_eval_max(kern) && cap == n;
   if (grad && !small && Xinv.n < nn) {
     size_t half = (size_t)((n + 1) / 2) * ((n + 1) / 2);
     if (Xinv.alloc(nn) != cudaSuccess || scratch.alloc(std::max<size_t>(half, 1)) != cudaSuccess) {

@@ -53,10 +53,16 @@ cudaError_t cross_contract(const HostKernel& k, const double* z, long long ldz, 
 cudaError_t grad_finalize(const HostKernel& k, const double* partials, int blocks, const int* slot_param_dev,
                           double scale, double noise_coef, double* grad, DevStatus* st, cudaStream_t s);
 
-// One evaluation of at most SMALL_EVAL_N points in one launch (batch.cu): x is
+// One evaluation of at most small_eval_max points in one launch (batch.cu): x is
 // n×d with leading dimension n; res[0] = log-det, res[1] = yᵀα, res[2 ..] the
 // gradient; α to alpha.  A failed factor or a non-finite kernel value goes to st.
-constexpr int SMALL_EVAL_N = 128;
+//
+// One block of 128 points; with more than 16 ARD dimensions one 64×64 tile: the
+// gradient's 64 values a thread lie in local memory there, and from the second tile
+// on one CTA takes longer over them than the launches cost (µs, one launch /
+// separate ones: d = 17 n = 65 388 / 264, n = 128 536 / 271; d = 32 n = 65 600 / 370,
+// n = 128 838 / 374; at n = 64 one launch takes 216 and 316).
+inline int small_eval_max(const HostKernel& k) { return k.ard_d > 16 ? 64 : 128; }
 cudaError_t small_eval(const HostKernel& k, const double* x, const double* y, int n, double diag_add, double noise,
                        const int* slot_param, double* alpha, double* res, DevStatus* st, cudaStream_t s);
 
