@@ -160,16 +160,9 @@ __global__ void __launch_bounds__(FD_THREADS) tri_inv_blocks_kernel(const double
 static size_t fast_diag_smem(int nb) { (void)nb; return diag_block_smem(); }
 
 static cudaError_t diag_attrs() {
-  static bool done = false;
-  if (done) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)fast_diag_smem(NB));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(tri_inv_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)fast_diag_smem(NB));
-  if (e != cudaSuccess) return e;
-  done = true;
-  return cudaSuccess;
+  static SmemAllowed factor, inverse;
+  const cudaError_t e = factor((const void*)potrf_diag_kernel, fast_diag_smem(NB));
+  return e != cudaSuccess ? e : inverse((const void*)tri_inv_blocks_kernel, fast_diag_smem(NB));
 }
 
 #define CK(x)                                \
@@ -346,12 +339,8 @@ static cudaError_t launch_chain(void (*kernel)(Params...), dim3 grid, dim3 block
 
 template <int TM>
 static cudaError_t panel_gemm_launch(const PanelGemmArgs& g, cudaStream_t s, bool chained) {
-  static bool attr = false;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(panel_gemm_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)panel_gemm_smem<TM>()));
-    attr = true;
-  }
+  static SmemAllowed allowed;
+  CK(allowed((const void*)panel_gemm_kernel<TM>, panel_gemm_smem<TM>()));
   if (chained)
     return launch_chain(panel_gemm_kernel<TM>, dim3(ceil_div(g.M, TM)), dim3(256), panel_gemm_smem<TM>(), s, g);
   GPRX_LAUNCH(panel_gemm_kernel<TM>, ceil_div(g.M, TM), 256, panel_gemm_smem<TM>(), s, g);

@@ -18,6 +18,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "smem_allowed.h"
 
 namespace gprx {
 
@@ -307,12 +308,9 @@ template <int BM, int BN, int BK, int WM, int WN, int STAGES, bool TA, bool TB>
 cudaError_t launch_dgemm(const GemmParams& p, int batch, cudaStream_t stream) {
   using Cfg = GemmCfg<BM, BN, BK, WM, WN, STAGES, TA, TB>;
   auto kern = dgemm_kernel<BM, BN, BK, WM, WN, STAGES, TA, TB>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SmemAllowed allowed;
+  const cudaError_t e = allowed((const void*)kern, Cfg::SMEM);
+  if (e != cudaSuccess) return e;
   if (p.M <= 0 || p.N <= 0) return cudaSuccess;
   int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
   int nblocks;
