@@ -91,8 +91,7 @@ GemmParams gemm_params(int M, int N, int K, const double* A, long long lda, cons
   p.split_stride = 0;
   p.status = st;
   p.strideA = p.strideB = p.strideC = 0;
-  p.max_ctas = 0;
-  p.splits_tiles = 0;
+  p.tiles = 0;
   return p;
 }
 

@@ -52,8 +52,7 @@ struct GemmParams {
   const DevStatus* status;
   // batched: pointer strides per blockIdx.z when splits == 1 and batch > 1
   long long strideA, strideB, strideC;
-  int max_ctas;             // > 0: at most this many CTAs, each looping over tiles
-  int splits_tiles;         // set by the launcher: tile count
+  int tiles;                // set by the launcher: output tiles
 };
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {
@@ -96,24 +95,18 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES, TA, TB>::T
   using Cfg = GemmCfg<BM, BN, BK, WM, WN, STAGES, TA, TB>;
   extern __shared__ __align__(16) double smem[];
   if (dev_failed(p.status)) return;
-  const int ntiles_total = p.max_ctas > 0 ? p.max_ctas : 0;  // set by the launcher when capped
-  for (int tile_idx = blockIdx.x;; tile_idx += gridDim.x) {
-  if (p.max_ctas > 0) {
-    if (tile_idx >= p.splits_tiles) break;
-    __syncthreads();  // the previous tile's shared-memory reads are done
-  } else if (tile_idx != (int)blockIdx.x) {
-    break;
-  }
-  (void)ntiles_total;
 
   // ---- which output tile ----
+  // (one tile a CTA; as a loop it compiles to 150 registers where straight code takes
+  // 133, and is 0.5 to 1% faster at n = 8192 and in the Sgpr products)
+  for (int tile_idx = blockIdx.x; tile_idx < p.tiles; tile_idx += gridDim.x) {
   int tile_m, tile_n;
   const int tiles_m = (p.M + BM - 1) / BM;
   if (p.mode & GEMM_LOWER_TILES) {
     // tile_idx enumerates (tm, tn) with the tile not strictly above the
     // diagonal; when row0 == col0 and BM == BN that is tn ≤ tm.
     // tiles with the longest k range first: the last wave is then of short ones
-    int idx = (p.mode & GEMM_K_TO_COL) ? p.splits_tiles - 1 - tile_idx : tile_idx;
+    int idx = (p.mode & GEMM_K_TO_COL) ? p.tiles - 1 - tile_idx : tile_idx;
     // general enumeration: walk columns; tile (tm, tn) is kept when its last
     // global row ≥ its first global column.
     const int tiles_n = (p.N + BN - 1) / BN;
@@ -130,7 +123,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES, TA, TB>::T
       idx -= cnt;
     }
     if (tile_m < 0) return;
-  } else if ((p.mode & GEMM_K_TO_ROW) && p.splits_tiles <= GEMM_ROWS_FIRST_TILES) {
+  } else if ((p.mode & GEMM_K_TO_ROW) && p.tiles <= GEMM_ROWS_FIRST_TILES) {
     const int tiles_n = (p.N + BN - 1) / BN;  // longest k range (last rows) first
     tile_m = tiles_m - 1 - tile_idx / tiles_n;
     tile_n = tile_idx % tiles_n;
@@ -300,7 +293,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES, TA, TB>::T
         C[row + (long long)col * p.ldc] = v;
       }
   }
-  }  // tile loop
+  }
 }
 
 // Host-side launcher for one configuration.
@@ -327,8 +320,7 @@ cudaError_t launch_dgemm(const GemmParams& p, int batch, cudaStream_t stream) {
     nblocks = tiles_m * tiles_n;
   }
   GemmParams q = p;
-  q.splits_tiles = nblocks;
-  if (p.max_ctas > 0 && nblocks > p.max_ctas) nblocks = p.max_ctas;
+  q.tiles = nblocks;
   dim3 grid(nblocks, 1, (p.mode & GEMM_SPLIT_K) ? p.splits : batch);
   kern<<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(q);
   count_launch();
