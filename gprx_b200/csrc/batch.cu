@@ -361,7 +361,9 @@ __device__ void cta_trtri(const Work& w, int n, long long ld, double* smem, int 
 // their registers into local memory (64 ARD problems of 200 to 256 points 667
 // against 613 µs).  Nothing but x, y and the results touches global memory.  α goes to
 // `alpha` (n values), the gradient's slot sums to `slots`; *logdet and *quad are
-// set in every thread.  Returns −1, the failing column, or SMALL_NONFINITE.
+// set in every thread.  clk (or null): the SM's clock at the start, after the fill,
+// the factor with the block's inverse, K⁻¹ and the gradient.  Returns −1, the
+// failing column, or SMALL_NONFINITE.
 constexpr int SMALL_NONFINITE = -2;
 inline size_t tile_smem() {
   return (size_t)(2 * GPRX_MAX_DIM * FT_B + 2 * FT_B + (BT / 32) * 64) * sizeof(double);
@@ -370,7 +372,12 @@ inline size_t small_smem() { return diag_block_smem() + tile_smem() + 2 * NB_DIA
 
 template <int ARD_D, int NL>
 __device__ __noinline__ int cta_small(const KTree& tree, const double* x, const double* y, int n, double diag_add, double* smem,
-                         int* flag_sh, double* red, double* slots, double* alpha, double* logdet, double* quad) {
+                         int* flag_sh, double* red, double* slots, double* alpha, double* logdet, double* quad,
+                         long long* clk = nullptr) {
+  auto mark = [&](int k) {
+    if (clk && threadIdx.x == 0) clk[k] = clock64();
+  };
+  mark(0);
   double* s = smem;
   double* tmp = s + NB_DIAG * FLS;
   double* ldiag = tmp + TMP_DOUBLES + NB_DIAG;
@@ -380,9 +387,11 @@ __device__ __noinline__ int cta_small(const KTree& tree, const double* x, const 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int np = (n + LF - 1) / LF, npad = np * LF;
   if (!cta_fill_lower<ARD_D, NL>(tree, x, n, s, FLS, diag_add, tiles, flag_sh)) return SMALL_NONFINITE;
+  mark(1);
   diag_block_pad(s, n);
   const int f = diag_block_core(nullptr, 0, 0, n, nullptr, false, smem, flag_sh);
   if (f >= 0) return f;
+  mark(2);
   double acc = 0.0;
   for (int i = tid; i < n; i += BT) acc += log(ldiag[i]);
   *logdet = 2.0 * block_sum(acc, red);
@@ -456,7 +465,9 @@ __device__ __noinline__ int cta_small(const KTree& tree, const double* x, const 
       }
   }
   __syncthreads();
+  mark(3);
   cta_grad<ARD_D, NL>(tree, x, n, s, FLS, av, tiles, slots);
+  mark(4);
   return -1;
 }
 
@@ -473,8 +484,8 @@ __device__ inline void slots_to_grad(const double* slots, int ns, const int* slo
 }
 
 // One evaluation of one exact problem of at most 128 points in one launch: the
-// log-det, yᵀα and the gradient to res[0], res[1], res[2 ..], α to alpha.
-// Latency-bound: the pivots' chain and a few passes over one block.  As 12
+// log-det, yᵀα and the gradient to res[0], res[1], res[2 ..], α to alpha, the
+// clocks of its four stages to res[SMALL_STAGE_AT ..].  Latency-bound: the pivots' chain and a few passes over one block.  As 12
 // launches (fill, diagonal step, log-det, copy, two products, two vector
 // products, a dot product, K⁻¹, gradient, its sums) n = 64 took 108 µs.
 template <int ARD_D, int NL>
@@ -486,9 +497,11 @@ __global__ void __launch_bounds__(BT, 1) small_eval_kernel(const __grid_constant
   __shared__ int flag_sh;
   __shared__ double red[32];
   __shared__ double slots[64];
+  __shared__ long long clk[5];
   if (dev_failed(st)) return;
   double logdet, quad;
-  const int f = cta_small<ARD_D, NL>(tree, x, y, n, diag_add, smem, &flag_sh, red, slots, alpha, &logdet, &quad);
+  const int f =
+      cta_small<ARD_D, NL>(tree, x, y, n, diag_add, smem, &flag_sh, red, slots, alpha, &logdet, &quad, clk);
   if (threadIdx.x != 0) return;
   if (f != -1) {
     dev_fail(st, f == SMALL_NONFINITE ? GPRX_NONFINITE_KERNEL : GPRX_CHOLESKY_FAILED, f < 0 ? 0 : f);
@@ -496,6 +509,7 @@ __global__ void __launch_bounds__(BT, 1) small_eval_kernel(const __grid_constant
   }
   res[0] = logdet;
   res[1] = quad;
+  for (int k = 0; k < 4; ++k) res[SMALL_STAGE_AT + k] = (double)(clk[k + 1] - clk[k]);
   slots_to_grad(slots, GRAD_SLOTS_LEAF + (ARD_D > 0 ? ARD_D : 1) + 1, slot_param, noise, p, res + 2);
 }
 

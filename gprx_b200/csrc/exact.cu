@@ -879,7 +879,10 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
 gprx_status ExactState::stage_times(double* out5) {
   if (!ev_recorded) return set_error(GPRX_INVALID_CONFIG, "no evaluation recorded");
   float ms;
-  if (ev_single) {  // one launch: all of it under the fill's entry
+  if (ev_single) {  // one launch: its time divided as its own clock says
+    double clk[4];
+    GPRX_CUDA_TRY(cudaMemcpyAsync(clk, res.p + SMALL_STAGE_AT, sizeof(clk), cudaMemcpyDeviceToHost, stream));
+    GPRX_CUDA_TRY(cudaStreamSynchronize(stream));
     GPRX_CUDA_TRY(cudaEventElapsedTime(&ms, ev[0], ev[4]));
     out5[0] = out5[4] = ms;
     out5[1] = out5[2] = out5[3] = 0.0;

@@ -55,7 +55,10 @@ cudaError_t grad_finalize(const HostKernel& k, const double* partials, int block
 
 // One evaluation of at most small_eval_max points in one launch (batch.cu): x is
 // n×d with leading dimension n; res[0] = log-det, res[1] = yᵀα, res[2 ..] the
-// gradient; α to alpha.  A failed factor or a non-finite kernel value goes to st.
+// gradient, res[SMALL_STAGE_AT ..] the SM clocks of fill, factor, inverse and
+// gradient (no tree has so many parameters that they meet); α to alpha.  A failed
+// factor or a non-finite kernel value goes to st.
+constexpr int SMALL_STAGE_AT = 60;
 //
 // One block of 128 points; with more than 16 ARD dimensions one 64×64 tile: the
 // gradient's 64 values a thread lie in local memory there, and from the second tile

@@ -307,7 +307,9 @@ gprx_status gprx_exact_fit(gprx_exact* h, const gprx_lbfgs_options* opt, gprx_fi
 gprx_status gprx_exact_fit_trust_region(gprx_exact* h, const gprx_trust_region_options* opt,
                                         gprx_fit_report* report);
 /* Per-stage device time of the last eval in milliseconds:
- * [fill, factor, inverse, gradient, total] (the reference's insert-stages idea). */
+ * [fill, factor, inverse, gradient, total] (the reference's insert-stages idea).
+ * An evaluation of one launch (at most 128 points) divides its time by the clock
+ * of the SM that ran it. */
 gprx_status gprx_exact_stage_times(gprx_exact* h, double* out5);
 
 /* The CUDA stream (a cudaStream_t) the handle enqueues its work on, so a
