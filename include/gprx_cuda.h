@@ -472,7 +472,8 @@ gprx_status gprx_batch_stream(gprx_batch* h, void** stream);
  * 2: 32×64×32, 3: 32×32×16).  The first gprx_batch_eval / gprx_batch_fit
  * autotunes it: every class present is timed with every shape on a sample of
  * its problems and the fastest is kept (cached per device and kernel tree
- * for the life of the process).  Every shape gives the same results bit for
+ * for the life of the process; the classes up to n = 128 run in one block
+ * whatever the shape and are timed by gprx_batch_autotune only).  Every shape gives the same results bit for
  * bit.  gprx_batch_autotune re-tunes at the given θ (n_problems × p);
  * gprx_batch_set_schedule fixes the shapes and turns tuning off;
  * gprx_batch_schedule reads the shapes, the tuning times (ms per launch,
