@@ -844,11 +844,16 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
   } else if (!factor_ok || !alpha_ok) {
     if ((st = factor_current()) != GPRX_OK) return st;
   }
-  const int qc_max = (int)std::max<long long>(1, std::min<long long>((long long)q, (1LL << 27) / std::max(n, 1)));
+  // chunks whose results fit a pinned block that is kept for reuse (pool.cpp)
+  const int qc_max = (int)std::max<long long>(
+      1, std::min<long long>({(long long)q, (1LL << 27) / std::max(n, 1), (long long)PINNED_MAX_BLOCK / 16}));
   if (qbuf.ensure((size_t)ld * qc_max) != cudaSuccess || qx.ensure((size_t)qc_max * (d + 3)) != cudaSuccess)
     return set_error(GPRX_OUT_OF_MEMORY, "predict scratch");
-  GPRX_CUDA_TRY(pred_h.ensure(2 * (size_t)qc_max));
-  double* const hm = pred_h.p;
+  // the handle keeps the pinned block of small calls only
+  HostPinned<double> large{lane};
+  HostPinned<double>& block = qc_max <= PRED_KEEP ? pred_h : large;
+  GPRX_CUDA_TRY(block.ensure(2 * (size_t)qc_max));
+  double* const hm = block.p;
   // one route for the whole call: a query's bits do not depend on its chunk
   const int cls = solve_class(n, (long long)q);
   const double kss = kern.diag_value();
