@@ -36,7 +36,6 @@ namespace {
 constexpr size_t POOL_KEEP = (size_t)1 << 30;
 constexpr size_t POOL_MAX_BLOCK = (size_t)256 << 20;  // larger buffers go to cudaMalloc
 constexpr size_t PINNED_KEEP = (size_t)8 << 20;
-constexpr size_t PINNED_MAX_BLOCK = (size_t)1 << 20;
 constexpr size_t STREAM_KEEP = 16;
 
 struct DevicePool {

@@ -36,7 +36,17 @@ class Lane {
 cudaError_t device_alloc(void** out, size_t bytes, int* device);
 void device_free(void* ptr, size_t bytes, int device, const Lane& lane);
 
-// Pinned host memory; pinned_free takes the size asked for.
+// One spare block an owner: a buffer it will want again but can do without.  All
+// spares of a device are freed before an allocation there fails, and what goes
+// beyond SPARE_KEEP bytes in all is freed at once.
+void spare_keep(const void* owner, void* ptr, size_t bytes, int device, const Lane& lane);
+// The owner's spare of at least *bytes (*bytes and *device receive its own), or null.
+void* spare_take(const void* owner, size_t* bytes, int* device);
+void spare_drop(const void* owner);
+
+// Pinned host memory; pinned_free takes the size asked for and keeps blocks of at
+// most PINNED_MAX_BLOCK bytes for reuse.
+constexpr size_t PINNED_MAX_BLOCK = (size_t)1 << 20;
 cudaError_t pinned_alloc(void** out, size_t bytes);
 void pinned_free(void* ptr, size_t bytes, const Lane& lane);
 
