@@ -889,8 +889,9 @@ gprx_status ExactState::stage_times(double* out5) {
     GPRX_CUDA_TRY(cudaMemcpyAsync(clk, res.p + SMALL_STAGE_AT, sizeof(clk), cudaMemcpyDeviceToHost, stream));
     GPRX_CUDA_TRY(cudaStreamSynchronize(stream));
     GPRX_CUDA_TRY(cudaEventElapsedTime(&ms, ev[0], ev[4]));
-    out5[0] = out5[4] = ms;
-    out5[1] = out5[2] = out5[3] = 0.0;
+    const double sum = clk[0] + clk[1] + clk[2] + clk[3];
+    for (int i = 0; i < 4; ++i) out5[i] = ms * clk[i] / sum;
+    out5[4] = ms;
     return GPRX_OK;
   }
   for (int i = 0; i < 4; ++i) {
