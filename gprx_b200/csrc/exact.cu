@@ -24,6 +24,7 @@ namespace gprx {
 
 ExactState::~ExactState() {
   lane.close();
+  spare_drop(this);
   for (auto& e : ev)
     if (e) cudaEventDestroy(e);
 }

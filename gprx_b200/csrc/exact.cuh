@@ -138,8 +138,8 @@ struct ExactState {
   // op leaves the LDLT, α and the jitter as they were
   // (with_llt_view, src/gpr/online.rs:1151-1185).
   DevBuf<double> ldlt_keep{lane}, alpha_keep{lane};
-  DevBuf<double> spare_A{lane}, spare_x{lane}, spare_y{lane};  // a delete writes here, then swaps
-  DevBuf<double> r1{lane};                         // its vectors: p, β, new D, per-block sums
+  DevBuf<double> spare_x{lane}, spare_y{lane};  // a delete writes here, then swaps
+  DevBuf<double> r1{lane};  // its vectors: p, β, new D, per-block sums (n²/128 values at most)
   gprx_status with_llt_view(const std::function<gprx_status()>& op);
   gprx_status online_insert(const double* xnew, double ynew, uint64_t* id);
   gprx_status online_delete(uint64_t id);

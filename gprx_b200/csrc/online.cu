@@ -277,7 +277,8 @@ gprx_status ExactState::online_delete(uint64_t id) {
   gprx_status st;
   if ((st = reset_status()) != GPRX_OK) return st;
   const int row0 = (idx + 1) / NB * NB, len = n - row0;  // whole blocks from the first trailing row
-  if (spare_A.ensure((size_t)ld * cap) != cudaSuccess || spare_x.ensure((size_t)cap * d) != cudaSuccess ||
+  DevBuf<double> nA{lane};  // the compacted factor, in the last delete's spare if it is still there
+  if (nA.take_spare(this, (size_t)ld * cap) != cudaSuccess || spare_x.ensure((size_t)cap * d) != cudaSuccess ||
       spare_y.ensure(cap) != cudaSuccess ||
       r1.ensure((size_t)std::max(len, 1) * (3 + ceil_div(std::max(len, 1), NB))) != cudaSuccess)
     return set_error(GPRX_OUT_OF_MEMORY, "online delete scratch");
@@ -301,15 +302,16 @@ gprx_status ExactState::online_delete(uint64_t id) {
                 status.p);
   }
   GPRX_LAUNCH(ldlt_delete_kernel, dim3(ceil_div(n, DEL_ROWS), ceil_div(n, NB)), DEL_ROWS, 0, stream, A.p, ld, n, idx,
-              row0, p, beta, dnew, prefix, (long long)len, spare_A.p, ld, status.p);
+              row0, p, beta, dnew, prefix, (long long)len, nA.p, ld, status.p);
   GPRX_LAUNCH(drop_row_kernel, ceil_div((long long)(n - 1) * d, 256) + 1, 256, 0, stream, x.p, cap, n, d, idx,
               spare_x.p, cap);
   GPRX_LAUNCH(drop_row_kernel, ceil_div(n, 256) + 1, 256, 0, stream, y.p, cap, n, 1, idx, spare_y.p, cap);
   DevStatus ds;
   if ((st = read_status(&ds)) != GPRX_OK) return st;
   if (ds.code != GPRX_OK) return status_to_error(ds, 0.0, n, GPRX_STAGE_ONLINE_DELETE);
-  std::swap(A.p, spare_A.p);
-  std::swap(A.n, spare_A.n);
+  std::swap(A.p, nA.p);
+  std::swap(A.n, nA.n);
+  nA.keep_spare(this);
   std::swap(x.p, spare_x.p);
   std::swap(x.n, spare_x.n);
   std::swap(y.p, spare_y.p);

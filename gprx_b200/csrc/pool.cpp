@@ -11,6 +11,9 @@
 //    a free first waits for its owner's streams (Lane) and drains it again: then
 //    the pool gives what it holds above POOL_KEEP back to the driver.  All of its
 //    unused memory goes back when an allocation fails.
+//  * an online model's second factor-sized buffer waits here between deletes
+//    (spare_keep), so that it is there for the next one and for nobody's loss: all
+//    of them hold SPARE_KEEP at most, and an allocation that would fail takes them.
 //  * pinned blocks and idle streams are kept in small bounded lists (PINNED_KEEP
 //    bytes, STREAM_KEEP streams of a kind); what does not fit is freed.
 //
@@ -35,6 +38,7 @@ namespace {
 
 constexpr size_t POOL_KEEP = (size_t)1 << 30;
 constexpr size_t POOL_MAX_BLOCK = (size_t)256 << 20;  // larger buffers go to cudaMalloc
+constexpr size_t SPARE_KEEP = (size_t)4 << 30;
 constexpr size_t PINNED_KEEP = (size_t)8 << 20;
 constexpr size_t STREAM_KEEP = 16;
 
@@ -45,9 +49,17 @@ struct DevicePool {
   std::vector<cudaStream_t> idle[2];  // by priority: normal, high
 };
 
+struct SpareBlock {
+  void* ptr;
+  size_t bytes;
+  int device;
+};
+
 struct Pools {
   std::mutex mu;
   std::map<int, DevicePool> dev;
+  std::map<const void*, SpareBlock> spare;  // by owner
+  size_t spare_bytes = 0;
   std::map<size_t, std::vector<void*>> pinned;  // by size class
   size_t pinned_bytes = 0;
 };
@@ -85,6 +97,39 @@ DevicePool* device_pool(Pools& p, int device) {
   return d.pool ? &d : nullptr;
 }
 
+// Frees a block that nothing uses.
+void free_idle(void* ptr, size_t bytes, int device) {
+  if (!ptr) return;
+  cudaStream_t stream = nullptr;
+  {
+    Pools& p = pools();
+    std::lock_guard<std::mutex> lock(p.mu);
+    if (DevicePool* d = device_pool(p, device)) stream = d->stream;
+  }
+  cudaError_t e;
+  if (!stream || bytes > POOL_MAX_BLOCK) e = cudaFree(ptr);
+  else if ((e = cudaFreeAsync(ptr, stream)) == cudaSuccess) e = cudaStreamSynchronize(stream);  // past POOL_KEEP: to the driver
+  if (e != cudaSuccess) (void)cudaGetLastError();
+}
+
+// Removes the owner's spare block (of any owner with null; on `device` only unless −1)
+// from the list; ptr is null when there is none.
+SpareBlock spare_remove(const void* owner, int device) {
+  Pools& p = pools();
+  std::lock_guard<std::mutex> lock(p.mu);
+  for (auto it = owner ? p.spare.find(owner) : p.spare.begin(); it != p.spare.end(); ++it) {
+    if (device >= 0 && it->second.device != device) {
+      if (owner) break;
+      continue;
+    }
+    const SpareBlock b = it->second;
+    p.spare_bytes -= b.bytes;
+    p.spare.erase(it);
+    return b;
+  }
+  return {nullptr, 0, 0};
+}
+
 }  // namespace
 
 cudaError_t device_alloc(void** out, size_t bytes, int* device) {
@@ -107,8 +152,10 @@ cudaError_t device_alloc(void** out, size_t bytes, int* device) {
     if (e == cudaSuccess) return pooled ? cudaStreamSynchronize(stream) : e;
     (void)cudaGetLastError();
     *out = nullptr;
-    if (e != cudaErrorMemoryAllocation || !pool) break;
-    // what the pool holds unused goes back to the driver
+    if (e != cudaErrorMemoryAllocation) break;
+    // the spares, and what the pool holds unused, go back to the driver
+    for (SpareBlock b; (b = spare_remove(nullptr, *device)).ptr;) free_idle(b.ptr, b.bytes, b.device);
+    if (!pool) continue;
     cudaStreamSynchronize(stream);
     cudaMemPoolTrimTo(pool, 0);
   }
@@ -116,19 +163,41 @@ cudaError_t device_alloc(void** out, size_t bytes, int* device) {
 }
 
 void device_free(void* ptr, size_t bytes, int device, const Lane& lane) {
+  // work that may use it could not be waited for: nobody else gets it
+  if (ptr && (lane.drain() || bytes > POOL_MAX_BLOCK)) free_idle(ptr, bytes, device);
+}
+
+void spare_keep(const void* owner, void* ptr, size_t bytes, int device, const Lane& lane) {
   if (!ptr) return;
-  cudaStream_t stream = nullptr;
+  spare_drop(owner);
+  if (!lane.drain()) return device_free(ptr, bytes, device, lane);
   {
     Pools& p = pools();
     std::lock_guard<std::mutex> lock(p.mu);
-    if (DevicePool* d = device_pool(p, device)) stream = d->stream;
+    if (p.spare_bytes + bytes <= SPARE_KEEP) {
+      p.spare[owner] = {ptr, bytes, device};
+      p.spare_bytes += bytes;
+      return;
+    }
   }
-  const bool idle = lane.drain();
-  cudaError_t e = cudaSuccess;
-  if (!stream || bytes > POOL_MAX_BLOCK) e = cudaFree(ptr);
-  else if (idle && (e = cudaFreeAsync(ptr, stream)) == cudaSuccess) e = cudaStreamSynchronize(stream);  // past POOL_KEEP: to the driver
-  // not idle: work that may use it could not be waited for, so nobody else gets it
-  if (e != cudaSuccess) (void)cudaGetLastError();
+  free_idle(ptr, bytes, device);
+}
+
+void* spare_take(const void* owner, size_t* bytes, int* device) {
+  const SpareBlock b = spare_remove(owner, -1);
+  if (!b.ptr) return nullptr;
+  if (b.bytes < *bytes) {
+    free_idle(b.ptr, b.bytes, b.device);
+    return nullptr;
+  }
+  *bytes = b.bytes;
+  *device = b.device;
+  return b.ptr;
+}
+
+void spare_drop(const void* owner) {
+  const SpareBlock b = spare_remove(owner, -1);
+  free_idle(b.ptr, b.bytes, b.device);
 }
 
 cudaError_t pinned_alloc(void** out, size_t bytes) {

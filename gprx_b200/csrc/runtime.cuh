@@ -52,6 +52,21 @@ struct DevBuf {
     p = nullptr;
     n = 0;
   }
+  // alloc, in the owner's spare block (pool.h) where it is there and large enough
+  cudaError_t take_spare(const void* owner, size_t count) {
+    reset();
+    size_t bytes = count * sizeof(T);
+    p = static_cast<T*>(spare_take(owner, &bytes, &device));
+    if (!p) return alloc(count);
+    n = bytes / sizeof(T);
+    return cudaSuccess;
+  }
+  // the buffer, which nothing uses any more, becomes the owner's spare block
+  void keep_spare(const void* owner) {
+    spare_keep(owner, p, n * sizeof(T), device, lane);
+    p = nullptr;
+    n = 0;
+  }
 };
 
 // Pinned host scratch.
