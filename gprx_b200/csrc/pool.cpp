@@ -167,10 +167,9 @@ void device_free(void* ptr, size_t bytes, int device, const Lane& lane) {
   if (ptr && (lane.drain() || bytes > POOL_MAX_BLOCK)) free_idle(ptr, bytes, device);
 }
 
-void spare_keep(const void* owner, void* ptr, size_t bytes, int device, const Lane& lane) {
+void spare_keep(const void* owner, void* ptr, size_t bytes, int device) {
   if (!ptr) return;
   spare_drop(owner);
-  if (!lane.drain()) return device_free(ptr, bytes, device, lane);
   {
     Pools& p = pools();
     std::lock_guard<std::mutex> lock(p.mu);

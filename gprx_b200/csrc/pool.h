@@ -39,7 +39,8 @@ void device_free(void* ptr, size_t bytes, int device, const Lane& lane);
 // One spare block an owner: a buffer it will want again but can do without.  All
 // spares of a device are freed before an allocation there fails, and what goes
 // beyond SPARE_KEEP bytes in all is freed at once.
-void spare_keep(const void* owner, void* ptr, size_t bytes, int device, const Lane& lane);
+// Nothing uses the block any more: its owner has waited for its work.
+void spare_keep(const void* owner, void* ptr, size_t bytes, int device);
 // The owner's spare of at least *bytes (*bytes and *device receive its own), or null.
 void* spare_take(const void* owner, size_t* bytes, int* device);
 void spare_drop(const void* owner);

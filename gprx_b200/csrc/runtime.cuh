@@ -61,9 +61,9 @@ struct DevBuf {
     n = bytes / sizeof(T);
     return cudaSuccess;
   }
-  // the buffer, which nothing uses any more, becomes the owner's spare block
+  // the buffer, whose work has been waited for, becomes the owner's spare block
   void keep_spare(const void* owner) {
-    spare_keep(owner, p, n * sizeof(T), device, lane);
+    spare_keep(owner, p, n * sizeof(T), device);
     p = nullptr;
     n = 0;
   }
