@@ -22,6 +22,7 @@
 // two accumulators, whichever CTA does it.
 
 #include <algorithm>
+#include <atomic>
 
 #include "dense_f64.cuh"
 
@@ -31,7 +32,6 @@ namespace {
 
 constexpr int TS_THREADS = 256;
 constexpr int TS_LD = NB + 4;  // ≡ 4 mod 16 doubles: conflict-free fragments
-constexpr int TS_MAX_CLUSTER = 16;
 constexpr int TS_SMEM_MAX = 227 * 1024;
 
 struct TriSolveArgs {
@@ -464,47 +464,54 @@ cudaError_t ts_launch(void (*kern)(Args), const Args& g, int ctas, size_t smem, 
   return cudaLaunchKernelEx(&cfg, kern, g);
 }
 
-// Whether the device can hold a cluster of 16 CTAs of one SM each (non-portable).
-bool ts_cluster16() {
-  static int cached[64] = {0};  // 0 unknown, 1 yes, 2 no; the same answer from every thread
+// Clusters of 2^lc CTAs that the current device holds at once (one CTA takes an SM;
+// a cluster lies in one GPC, so there are fewer than SMs / CTAs of them: 16 of 8 and
+// 7 of 16).  0: no such cluster.
+int ts_resident(int lc) {
+  static std::atomic<int> cached[64][5];  // the count plus one; the same answer from every thread
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  if (cached[dev] == 0) {
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::atomic<int>& known = cached[dev][lc];
+  if (known.load(std::memory_order_relaxed) == 0) {
     auto kern = tri_solve_kernel<false, 1>;
     int clusters = 0;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(16);
+    cfg.gridDim = dim3(1u << lc);
     cfg.blockDim = dim3(TS_THREADS);
     cfg.dynamicSmemBytes = TS_SMEM_MAX;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 16;
+    at[0].val.clusterDim.x = 1u << lc;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX) == cudaSuccess &&
-                    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0;
-    if (!ok) (void)cudaGetLastError();
-    cached[dev] = ok ? 1 : 2;
+                    (lc < 4 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+                    cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess;
+    if (!ok) {
+      (void)cudaGetLastError();
+      clusters = 0;
+    }
+    known.store(clusters + 1, std::memory_order_relaxed);
   }
-  return cached[dev] == 1;
+  return known.load(std::memory_order_relaxed) - 1;
 }
 
 // (NT, C) of a solve: 16-column strips from nine columns on; the largest
-// cluster that keeps every strip resident at once (148 SMs) and has a block
-// for every CTA, as far as the owned blocks' sums fit in shared memory.
-bool ts_plan(int n, int q, int* NT, int* C) {
+// cluster of which the device holds one for every strip at once and that has a
+// block for every CTA, as far as the owned blocks' sums fit in shared memory.
+// *held: every strip is resident.
+bool ts_plan(int n, int q, int* NT, int* C, bool* held) {
   const int nblk = ceil_div(n, NB);
-  const int cmax = ts_cluster16() ? TS_MAX_CLUSTER : 8;
   for (int nt = q > 8 ? 2 : 1; nt >= 1; --nt) {
     const int strips = ceil_div(q, 8 * nt);
-    int c = 1;
-    while (c * 2 <= cmax && c * 2 <= nblk && (long long)c * 2 * strips <= 148) c *= 2;
-    while (c < cmax && ts_smem(nt, ceil_div(nblk, c), q == 1) > TS_SMEM_MAX) c *= 2;
-    if (ts_smem(nt, ceil_div(nblk, c), q == 1) <= TS_SMEM_MAX) {
+    int lc = 0;
+    while (lc < 4 && (2 << lc) <= nblk && ts_resident(lc + 1) >= strips) ++lc;
+    while (lc < 4 && ts_smem(nt, ceil_div(nblk, 1 << lc), q == 1) > TS_SMEM_MAX && ts_resident(lc + 1) > 0) ++lc;
+    if (ts_smem(nt, ceil_div(nblk, 1 << lc), q == 1) <= TS_SMEM_MAX) {
       *NT = nt;
-      *C = c;
+      *C = 1 << lc;
+      *held = ts_resident(lc) >= strips;
       return true;
     }
   }
@@ -513,19 +520,29 @@ bool ts_plan(int n, int q, int* NT, int* C) {
 
 }  // namespace
 
-// One launch while the strips' reads of L are small: n·q ≤ 200 000, and one
-// right-hand side always.  Above, recursion with blocks of 512 rows up to
-// q = 1200 and of 256 rows from there on.  Measured (µs, one launch / 512 / 256 /
-// two GEMMs per 128 rows): n = 512, q = 500 37 / 37 / 45 / 94; n = 1000, q = 64
-// 61 / 83 / 108 / 193, 256 119 / 83 / 108 / 192, 1000 130 / 104 / 122 / 232, 2000
-// 255 / 192 / 176 / 281; n = 4096, q = 1 193 / – / – / 807, 64 328 / 478 / 579 /
-// 807, 256 1005 / 551 / 636 / 1011, 1500 – / 1627 / 1546 / 1881, 10000 – / 6887 /
-// 6785 / 7763.  From q = 16384 on the launch's L2 reads (n²/2 values for every
-// 16 columns) cost more than products of 128-row blocks with their inverses: an
-// Sgpr evaluation (m = 1024, q = 10⁶) takes 344 ms with blocks of 256, 307 ms so.
+// One launch while the device holds every strip's cluster at once and a CTA's own
+// blocks fold at most six 8-column tiles a step (SOLVE_OWN: then the chain of blocks,
+// not the folds, sets the pace), and one right-hand side always.  Else recursion
+// with blocks of 512 rows up to q = 1200 and of 256 rows from there on.  Measured
+// (a prediction, µs, one launch / 512): n = 1000, q = 64 112 / 134, 400 116 / 138;
+// n = 2000, q = 64 172 / 254, 200 186 / 261, 320 (eight tiles) 312 / 283; n = 4096,
+// q = 112 397 / 557, 160 (eight) 735 / 615; n = 8192, q = 48 844 / 1256, 64 (not held)
+// 1691 / 1255; n = 16384, q = 8 (eight) 3150 / 2739.  Up to 512 rows both are the one
+// launch, and the line lies where a prediction's sums by a CTA a column stop paying
+// (n = 256, q = 1200 78 / 67).  The solve alone (512 / 256 / two
+// GEMMs per 128 rows): n = 1000, q = 1000 104 / 122 / 232, 2000 192 / 176 / 281;
+// n = 4096, q = 1500 1627 / 1546 / 1881, 10000 6887 / 6785 / 7763.  From q = 16384 on
+// the launch's L2 reads (n²/2 values for every 16 columns) cost more than products of
+// 128-row blocks with their inverses: an Sgpr evaluation (m = 1024, q = 10⁶) takes
+// 344 ms with blocks of 256, 307 ms so.
+constexpr int SOLVE_OWN = 6;
 int solve_class(long long n, long long q) {
   int nt, c;
-  if (q == 1 || (n * q <= 200000 && ts_plan((int)n, (int)q, &nt, &c))) return SOLVE_FEW;
+  bool held;
+  if (q == 1) return SOLVE_FEW;
+  if (q <= 1200 && (n > 512 || n * q <= 200000) && ts_plan((int)n, (int)q, &nt, &c, &held) && held &&
+      nt * ceil_div(ceil_div((int)n, NB), c) <= SOLVE_OWN)
+    return SOLVE_FEW;
   return q <= 1200 ? SOLVE_MID : q <= 16384 ? SOLVE_WIDE : SOLVE_BULK;
 }
 
@@ -533,7 +550,8 @@ cudaError_t tri_solve(const double* L, long long ld, int n, const double* linv, 
                       bool trans, const DevStatus* st, cudaStream_t s) {
   if (n <= 0 || q <= 0) return cudaSuccess;
   int nt, c;
-  if (!ts_plan(n, q, &nt, &c)) return cudaErrorInvalidValue;
+  bool held;
+  if (!ts_plan(n, q, &nt, &c, &held)) return cudaErrorInvalidValue;
   const TriSolveArgs g{L, ld, n, linv, B, ldb, q, c, st};
   const int strips = ceil_div(q, 8 * nt);
   const size_t smem = ts_smem(nt, ceil_div(ceil_div(n, NB), c), q == 1);
@@ -545,9 +563,9 @@ cudaError_t tri_solve(const double* L, long long ld, int n, const double* linv, 
 cudaError_t tri_solve_vec(const double* L, long long ld, int n, const double* linv, double* b, bool trans,
                           const DevStatus* st, cudaStream_t s, double* prefix, long long ldp) {
   if (n <= 0) return cudaSuccess;
-  const int nblk = ceil_div(n, NB), cmax = ts_cluster16() ? TS_MAX_CLUSTER : 8;
+  const int nblk = ceil_div(n, NB);
   int c = 1;
-  while (c * 2 <= cmax && c * 2 <= nblk) c *= 2;
+  for (int lc = 1; lc <= 4 && (1 << lc) <= nblk && ts_resident(lc) > 0; ++lc) c = 1 << lc;
   const size_t smem = tv_smem(ceil_div(nblk, c));
   if (smem > TS_SMEM_MAX || (prefix && trans)) return cudaErrorInvalidValue;
   const TriVecArgs g{L, ld, n, linv, b, c, prefix, ldp, st};
