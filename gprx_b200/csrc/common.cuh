@@ -48,6 +48,9 @@ uint64_t launches();
     ::gprx::count_launch();                                            \
   } while (0)
 
+// SMs of the one device this is built for (grids and tile rules are sized by it)
+constexpr int B200_SMS = 148;
+
 // ---------------------------------------------------------------------------
 // kernel tree in sum-of-products form
 // ---------------------------------------------------------------------------

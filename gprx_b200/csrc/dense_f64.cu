@@ -52,7 +52,7 @@ static long long gemm_tiles(const GemmParams& p, int bm, int bn) {
 template <bool TA, bool TB>
 static cudaError_t dgemm_fill(const GemmParams& p, cudaStream_t s, int batch) {
   const int z = (p.mode & GEMM_SPLIT_K) ? p.splits : batch;
-  if (gemm_tiles(p, 64, 64) * z >= 4 * 148) return dgemm_wide<TA, TB>(p, s, batch);
+  if (gemm_tiles(p, 64, 64) * z >= 4 * B200_SMS) return dgemm_wide<TA, TB>(p, s, batch);
   return launch_dgemm<32, 64, 32, 16, 16, 4, TA, TB>(p, batch, s);
 }
 
@@ -352,7 +352,7 @@ static cudaError_t panel_gemm(int M, int N, int K, const double* A, long long ld
   if (M <= 0 || N <= 0) return cudaSuccess;
   if (N > NB || K > NB || K < 0) return cudaErrorInvalidValue;
   const PanelGemmArgs g{M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, lower ? 1 : 0, tri ? 1 : 0, st};
-  return M <= 16 * 148 ? panel_gemm_launch<16>(g, s, chained) : panel_gemm_launch<PG_TM>(g, s, chained);
+  return M <= 16 * B200_SMS ? panel_gemm_launch<16>(g, s, chained) : panel_gemm_launch<PG_TM>(g, s, chained);
 }
 
 // rows below the diagonal block up to which the chain uses dependent launch
@@ -486,7 +486,7 @@ __global__ void set_identity_kernel(double* X, long long ld, int n) {
 cudaError_t set_identity(double* X, long long ld, int n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   long long total = (long long)n * n;
-  int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
+  int blocks = (int)std::min<long long>((total + 255) / 256, (long long)B200_SMS * 16);
   GPRX_LAUNCH(set_identity_kernel, blocks, 256, 0, s, X, ld, n);
   return cudaGetLastError();
 }
@@ -677,16 +677,16 @@ static int rec_split(int n) { return ceil_div(ceil_div(n, 2), NB) * NB; }
 
 // The block a class's recursion ends with: one tri_solve launch up to so many
 // rows, or (SOLVE_BULK) one 128-row block times its inverse, in place.
-static int solve_leaf(int cls, int n) {
+static int solve_leaf(SolveClass cls, int n) {
   return cls == SOLVE_FEW ? n : cls == SOLVE_MID ? 512 : cls == SOLVE_WIDE ? 256 : NB;
 }
-static cudaError_t solve_block(int cls, const double* L, long long ld, int n, const double* linv, double* B,
+static cudaError_t solve_block(SolveClass cls, const double* L, long long ld, int n, const double* linv, double* B,
                                long long ldb, int q, bool trans, DevStatus* st, cudaStream_t s) {
   if (cls != SOLVE_BULK) return tri_solve(L, ld, n, linv, B, ldb, q, trans, st, s);
   return dgemm_inplace(trans, gemm_params(n, q, n, linv, NB, B, ldb, B, ldb, 1.0, 0.0, st), s);
 }
 
-cudaError_t trsm_lower(int cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+cudaError_t trsm_lower(SolveClass cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
                        int q, DevStatus* st, cudaStream_t s) {
   const int n1 = rec_split(n);
   if (n <= solve_leaf(cls, n) || n1 >= n) return solve_block(cls, L, ld, n, linv, B, ldb, q, false, st, s);
@@ -698,7 +698,7 @@ cudaError_t trsm_lower(int cls, const double* L, long long ld, int n, const doub
                     st, s);
 }
 
-cudaError_t trsm_lower_t(int cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+cudaError_t trsm_lower_t(SolveClass cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
                          int q, DevStatus* st, cudaStream_t s) {
   const int n1 = rec_split(n);
   if (n <= solve_leaf(cls, n) || n1 >= n) return solve_block(cls, L, ld, n, linv, B, ldb, q, true, st, s);

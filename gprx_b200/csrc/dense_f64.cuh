@@ -6,6 +6,7 @@
 
 #include "gemm_f64.cuh"
 #include "pool.h"
+#include "solve_class.h"
 
 namespace gprx {
 
@@ -65,18 +66,16 @@ struct EmuWork;
 // B (n×q, ldb) := L⁻¹ B   /   := L⁻ᵀ B, with L's diagonal block inverses: by
 // recursive halving (X1 from the top half, one update B2 −= L21 X1 with K = n/2,
 // then the bottom half; the transpose bottom half first) down to blocks that
-// tri_solve takes in one launch (SOLVE_BULK: to 128-row blocks).  The class (solve_class of the whole solve)
-// fixes where the recursion stops, and with it the bits of a column: they do
-// not depend on q within a class.
-enum SolveClass : int { SOLVE_FEW = 0, SOLVE_MID = 1, SOLVE_WIDE = 2, SOLVE_BULK = 3 };
-int solve_class(long long n, long long q);
+// tri_solve takes in one launch (SOLVE_BULK: to 128-row blocks).  The class
+// (solve_class of the whole solve) fixes where the recursion stops, and with it the
+// bits of a column: they do not depend on q within a class.
 cudaError_t trsm_lower(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
                        DevStatus* st, cudaStream_t s);
 cudaError_t trsm_lower_t(const double* L, long long ld, int n, const double* linv, double* B, long long ldb, int q,
                          DevStatus* st, cudaStream_t s);
-cudaError_t trsm_lower(int cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+cudaError_t trsm_lower(SolveClass cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
                        int q, DevStatus* st, cudaStream_t s);
-cudaError_t trsm_lower_t(int cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
+cudaError_t trsm_lower_t(SolveClass cls, const double* L, long long ld, int n, const double* linv, double* B, long long ldb,
                          int q, DevStatus* st, cudaStream_t s);
 
 // The same two solves (trans: L⁻ᵀ) in one launch of thread-block clusters

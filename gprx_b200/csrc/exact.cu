@@ -856,7 +856,7 @@ gprx_status ExactState::predict(const double* xs, uint64_t q, int kind, double* 
   GPRX_CUDA_TRY(block.ensure(2 * (size_t)qc_max));
   double* const hm = block.p;
   // one route for the whole call: a query's bits do not depend on its chunk
-  const int cls = solve_class(n, (long long)q);
+  const SolveClass cls = solve_class(n, (long long)q);
   const double kss = kern.diag_value();
   for (uint64_t c0 = 0; c0 < q; c0 += qc_max) {
     int qc = (int)std::min<uint64_t>(qc_max, q - c0);

@@ -9,7 +9,7 @@
 namespace gprx {
 
 constexpr int HESS_MAX_PARAMS = 40;   // GPRX_MAX_PARAMS
-constexpr int HESS_MAX_BLOCKS = 148 * 4;
+constexpr int HESS_MAX_BLOCKS = B200_SMS * 4;
 
 // θ index → (leaf, index among that leaf's parameters), for the kernel's
 // parameters (the noise is handled on the host).

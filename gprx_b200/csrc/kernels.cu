@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(FILL_THREADS) fill_cross_w_kernel(KTree t, con
 }
 
 static int fill_grid(long long ntiles) {
-  long long cap = 148LL * 8;
+  long long cap = (long long)B200_SMS * 8;
   return (int)std::max<long long>(1, std::min(ntiles, cap));
 }
 
@@ -454,7 +454,7 @@ cudaError_t fill_cross(const HostKernel& k, const double* x1, long long ldx1, in
 // device: gradient contraction
 // ---------------------------------------------------------------------------
 constexpr int GRAD_THREADS = 256;  // two blocks per SM for trees of ARD width ≤ 8 (128 registers, no spills)
-constexpr int GRAD_MAX_BLOCKS = 148 * 4;
+constexpr int GRAD_MAX_BLOCKS = B200_SMS * 4;
 
 int grad_max_blocks() { return GRAD_MAX_BLOCKS; }
 

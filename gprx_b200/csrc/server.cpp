@@ -45,10 +45,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/gprx_cuda.h"
-
-namespace gprx {
-int solve_class(long long n, long long q);  // dense_f64.cuh
-}
+#include "solve_class.h"
 
 namespace {
 
@@ -275,7 +272,7 @@ uint64_t gprx_server::pick(std::vector<uint64_t>& batch) {
   } else if (head->kind == PREDICT) {
     // consecutive predicts of the same kind share one launch, as long as the
     // merged call solves the way each would alone (the same bits either way)
-    const int cls = gprx::solve_class((long long)m.n, (long long)head->q);
+    const gprx::SolveClass cls = gprx::solve_class((long long)m.n, (long long)head->q);
     uint64_t total = head->q;
     while (!m.queue.empty()) {
       Request* nx = reqs[m.queue.front()].get();

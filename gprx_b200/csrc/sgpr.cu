@@ -300,7 +300,7 @@ __global__ void sgpr_finish_var_kernel(const double* an, const double* bn, int q
 }
 
 static int grid_for(long long work, int per) {
-  return (int)std::max<long long>(1, std::min<long long>((work + per - 1) / per, 148LL * 16));
+  return (int)std::max<long long>(1, std::min<long long>((work + per - 1) / per, (long long)B200_SMS * 16));
 }
 
 // ---------------------------------------------------------------------------

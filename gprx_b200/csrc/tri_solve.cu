@@ -536,7 +536,7 @@ bool ts_plan(int n, int q, int* NT, int* C, bool* held) {
 // 128-row blocks with their inverses: an Sgpr evaluation (m = 1024, q = 10⁶) takes
 // 344 ms with blocks of 256, 307 ms so.
 constexpr int SOLVE_OWN = 6;
-int solve_class(long long n, long long q) {
+SolveClass solve_class(long long n, long long q) {
   int nt, c;
   bool held;
   if (q == 1) return SOLVE_FEW;
