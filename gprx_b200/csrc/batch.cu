@@ -8,9 +8,10 @@
 // evaluation of ExactFit::value_and_gradient_into_fit (gprx
 // src/gpr/exact_fit.rs:319-341) in its own workspace:
 //   fill      lower K + (σn² + j) I                  (factor.rs:515-542)
-//   LLT       128-wide block columns: diagonal block factor + inverse in
-//             shared memory, panel P = A_below L_kk⁻ᵀ and trailing
-//             A22 −= P Pᵀ as in-CTA DMMA tile GEMMs  (chol.rs:141-167)
+//   LLT       128-wide block columns, left-looking: one product with all
+//             earlier panels, diagonal block factor + inverse in shared
+//             memory, panel P = A_below L_kk⁻ᵀ (in-CTA DMMA tile GEMMs;
+//             chol.rs:141-167)
 //   log-det   2 Σ ln L_ii                             (factor.rs:555-568)
 //   X = L⁻¹   block rows: X_i,<i = −L_ii⁻¹ (L_i,<i X_<i,<i)
 //   α         Xᵀ (X y);  K⁻¹ = Xᵀ X (lower)          (workspace.rs:395-425)

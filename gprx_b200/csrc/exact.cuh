@@ -58,7 +58,6 @@ struct ExactState {
   HostPinned<double> res_h{lane};
   HostPinned<DevStatus> status_h{lane};
   DevBuf<double> qbuf{lane}, qx{lane};  // predict scratch
-  static constexpr int PRED_KEEP = 4096;  // query points whose results' pinned block (64 KB) stays with the handle
   HostPinned<double> pred_h{lane};
   DevBuf<unsigned char> group_dev{lane};       // grouped-predict staging (this handle leads the group)
   HostPinned<unsigned char> group_host{lane};

@@ -93,6 +93,10 @@ struct HostPinned {
   }
 };
 
+// Query points of a prediction whose results' pinned block (256 KB) stays with the
+// handle; that of a larger call goes back to the shared list.
+constexpr int PRED_KEEP = 16384;
+
 inline long long round_ld(long long n) { return (n + 31) / 32 * 32; }
 
 bool all_finite(const double* v, size_t n);

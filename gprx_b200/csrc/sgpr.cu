@@ -335,7 +335,7 @@ struct SgprState {
   static constexpr int EMU_GROUP = 8 * EMU_PART_K;  // columns of n sliced at a time (8 parts in flight)
   bool use_emu() const { return opt.precision == GPRX_PRECISION_MIXED && n >= EMU_MIN_N; }
   gprx_status ensure_emu(EmuWork& w);
-  HostPinned<double> res_h{lane};
+  HostPinned<double> res_h{lane}, pred_h{lane};
   HostPinned<DevStatus> status_h{lane};
   FactorCtx fctx{lane};
   // host scalars of the assembly
@@ -838,7 +838,8 @@ gprx_status SgprState::predict(const double* xs, uint64_t q, int kind, double* m
   if (qbuf.ensure((size_t)ldm * qc_max) || qbuf2.ensure((size_t)ldm * qc_max) ||
       qx.ensure((size_t)qc_max * (d + 4)))
     return set_error(GPRX_OUT_OF_MEMORY, "predict scratch");
-  HostPinned<double> hm{lane};
+  HostPinned<double> large{lane};
+  HostPinned<double>& hm = qc_max <= PRED_KEEP ? pred_h : large;
   GPRX_CUDA_TRY(hm.ensure(2 * (size_t)qc_max));
   const double kss = kern.diag_value();
   if ((st = reset_status()) != GPRX_OK) return st;
