@@ -534,8 +534,13 @@ bool ts_plan(int n, int q, int* NT, int* C, bool* held) {
 // n = 4096, q = 1500 1627 / 1546 / 1881, 10000 6887 / 6785 / 7763.  From q = 16384 on
 // the launch's L2 reads (n²/2 values for every 16 columns) cost more than products of
 // 128-row blocks with their inverses: an Sgpr evaluation (m = 1024, q = 10⁶) takes
-// 344 ms with blocks of 256, 307 ms so.
+// 344 ms with blocks of 256, 307 ms so.  One block of at most 128 rows goes there from
+// q = 6000 on: the launch stages the block and its inverse for every 16 columns, the
+// product for every 64 (a sparse prediction with two solves, m = 64, µs, launch /
+// product: q = 4096 107 / 107, 8000 144 / 129, 16384 209 / 174; m = 16 107 / 103,
+// 143 / 120, 202 / 160).
 constexpr int SOLVE_OWN = 6;
+constexpr int SOLVE_ONE_BLOCK_Q = 6000;
 SolveClass solve_class(long long n, long long q) {
   int nt, c;
   bool held;
@@ -543,6 +548,7 @@ SolveClass solve_class(long long n, long long q) {
   if (q <= 1200 && (n > 512 || n * q <= 200000) && ts_plan((int)n, (int)q, &nt, &c, &held) && held &&
       nt * ceil_div(ceil_div((int)n, NB), c) <= SOLVE_OWN)
     return SOLVE_FEW;
+  if (n <= NB && q > SOLVE_ONE_BLOCK_Q) return SOLVE_BULK;
   return q <= 1200 ? SOLVE_MID : q <= 16384 ? SOLVE_WIDE : SOLVE_BULK;
 }
 

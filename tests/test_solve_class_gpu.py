@@ -17,7 +17,8 @@ PARAMS = np.array([math.log(v) for v in (0.7, 1.1, 1.6, 0.05)])
 
 # strips of 16 columns a cluster of 16, of 8, of 4, of 2; the last that one launch takes and the first that it does not
 @pytest.mark.parametrize("n,q", [(2000, 112), (2000, 113), (2000, 240), (2000, 257), (1500, 528), (1500, 700),
-                                 (3000, 112), (3000, 144), (513, 1200), (512, 390), (512, 391), (900, 1100)])
+                                 (3000, 112), (3000, 144), (513, 1200), (512, 390), (512, 391), (900, 1100),
+                                 (1, 6001), (77, 6001), (128, 6000), (128, 6001), (129, 6001)])
 def test_both_sides_match_oracle(n, q):
     d = 3
     rs = np.random.RandomState(n + q)
