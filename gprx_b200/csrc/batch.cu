@@ -159,8 +159,8 @@ __device__ inline void stage_points(const double* x, int n, int d, int i0, int j
 // lower K + diag_add I into A (ld); returns true when every value is finite
 // (trees of at most NL leaves)
 template <int ARD_D, int NL>
-__device__ __noinline__ bool cta_fill_lower(const KTree& t, const double* x, int n, double* A, long long ld, double diag_add,
-                               double* smem, int* flag_sh) {
+__device__ __noinline__ bool cta_fill_lower(const KTree& t, const double* x, int n, double* A, long long ld,
+                                            double diag_add, double* smem, int* flag_sh) {
   double* xi = smem;
   double* xj = smem + GPRX_MAX_DIM * FT_B;
   const int d = t.d, tid = threadIdx.x;
@@ -372,8 +372,8 @@ inline size_t tile_smem() {
 inline size_t small_smem() { return diag_block_smem() + tile_smem() + 2 * NB_DIAG * sizeof(double); }
 
 template <int ARD_D, int NL>
-__device__ __noinline__ int cta_small(const KTree& tree, const double* x, const double* y, int n, double diag_add, double* smem,
-                         int* flag_sh, double* red, double* slots, double* alpha, double* logdet, double* quad,
+__device__ __noinline__ int cta_small(const KTree& tree, const double* x, const double* y, int n, double diag_add,
+                                      double* smem, int* flag_sh, double* red, double* slots, double* alpha, double* logdet, double* quad,
                          long long* clk = nullptr) {
   auto mark = [&](int k) {
     if (clk && threadIdx.x == 0) clk[k] = clock64();
@@ -486,9 +486,10 @@ __device__ inline void slots_to_grad(const double* slots, int ns, const int* slo
 
 // One evaluation of one exact problem of at most 128 points in one launch: the
 // log-det, yᵀα and the gradient to res[0], res[1], res[2 ..], α to alpha, the
-// clocks of its four stages to res[SMALL_STAGE_AT ..].  Latency-bound: the pivots' chain and a few passes over one block.  As 12
-// launches (fill, diagonal step, log-det, copy, two products, two vector
-// products, a dot product, K⁻¹, gradient, its sums) n = 64 took 108 µs.
+// clocks of its four stages to res[SMALL_STAGE_AT ..].  Latency-bound: the pivots'
+// chain and a few passes over one block.  As 12 launches (fill, diagonal step,
+// log-det, copy, two products, two vector products, a dot product, K⁻¹, gradient, its
+// sums) n = 64 took 108 µs.
 template <int ARD_D, int NL>
 __global__ void __launch_bounds__(BT, 1) small_eval_kernel(const __grid_constant__ KTree tree, const double* x,
                                                            const double* y, int n, double diag_add, double noise,
@@ -1286,10 +1287,11 @@ static gprx_status noalloc_scratch_ptr(int dev, double** out) {
     double* p = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void**)&p, g_noalloc_scratch);
     if (e != cudaSuccess) return set_cuda_error(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
-    if ((e = allow_batch_eval(Form<0, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<0, KT_MAX_LEAVES>{})) != cudaSuccess ||
-        (e = allow_batch_eval(Form<4, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<4, KT_MAX_LEAVES>{})) != cudaSuccess ||
-        (e = allow_batch_eval(Form<8, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<8, KT_MAX_LEAVES>{})) != cudaSuccess ||
-        (e = allow_batch_eval(Form<16, KT_MAX_LEAVES>{})) != cudaSuccess)
+    constexpr int MANY = KT_MAX_LEAVES;
+    if ((e = allow_batch_eval(Form<0, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<0, MANY>{})) != cudaSuccess ||
+        (e = allow_batch_eval(Form<4, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<4, MANY>{})) != cudaSuccess ||
+        (e = allow_batch_eval(Form<8, 2>{})) != cudaSuccess || (e = allow_batch_eval(Form<8, MANY>{})) != cudaSuccess ||
+        (e = allow_batch_eval(Form<16, MANY>{})) != cudaSuccess)
       return set_cuda_error(e, "shared-memory attribute of the evaluation kernel");
     ptrs[dev] = p;
   }

@@ -59,8 +59,7 @@ cudaError_t grad_finalize(const HostKernel& k, const double* partials, int block
 // gradient (no tree has so many parameters that they meet); α to alpha.  A failed
 // factor or a non-finite kernel value goes to st.
 constexpr int SMALL_STAGE_AT = 60;
-//
-// One block of 128 points; with more than 16 ARD dimensions one 64×64 tile: the
+// The most points: one block of 128; with more than 16 ARD dimensions one 64×64 tile: the
 // gradient's 64 values a thread lie in local memory there, and from the second tile
 // on one CTA takes longer over them than the launches cost (µs, one launch /
 // separate ones: d = 17 n = 65 388 / 264, n = 128 536 / 271; d = 32 n = 65 600 / 370,

@@ -108,7 +108,8 @@ void free_idle(void* ptr, size_t bytes, int device) {
   }
   cudaError_t e;
   if (!stream || bytes > POOL_MAX_BLOCK) e = cudaFree(ptr);
-  else if ((e = cudaFreeAsync(ptr, stream)) == cudaSuccess) e = cudaStreamSynchronize(stream);  // past POOL_KEEP: to the driver
+  else if ((e = cudaFreeAsync(ptr, stream)) == cudaSuccess)
+    e = cudaStreamSynchronize(stream);  // what the pool holds past POOL_KEEP goes to the driver
   if (e != cudaSuccess) (void)cudaGetLastError();
 }
 
